@@ -10,7 +10,8 @@
 //   backward (data)  A[m = voxel][k = (tap, co)] = dy[voxel - tap][co]
 //                    B[n = ci][k]                = W[co][tap][ci]
 //   backward (weight) A[m = (tap, ci)][k = voxel] = x[voxel + tap][ci]
-//                    B[n = co][k = voxel]        = dy[voxel][co]   (split over K)
+//                    B[n = co][k = voxel]        = dy[voxel][co]   (split over K;
+//                    channel counts that k_wgrad.cu does not take)
 //
 // Activations are BF16 in planes of 8 channels, [C / 8][volume][z][y][x][8]
 // (C a multiple of 8; [volume][z][y][x][C] otherwise); a tap
@@ -24,7 +25,7 @@
 #include <algorithm>
 #include <mutex>
 
-#include "runtime.h"
+#include "net.h"
 #include "umma.cuh"
 
 namespace pyro {
@@ -841,6 +842,8 @@ inline int pad16(int n) { return (n + 15) / 16 * 16; }
 
 }  // namespace
 
+void* tensor_map_encoder() { return (void*)encode_fn(); }
+
 // y = conv(x, W) (+ bias, ReLU), or its transpose for backward data.
 cudaError_t conv3_forward(const bf16* x, int C, int nx, int ny, int nz, int nb, const bf16* w,
                           int Cout, const float* bias, int relu, bf16* y_bf16, float* y_f32,
@@ -873,6 +876,8 @@ cudaError_t conv3_backward_data(const bf16* dy, int Cout, int nx, int ny, int nz
 // by the caller).
 cudaError_t conv3_backward_weight(const bf16* x, int Cin, const bf16* dy, int Cout, int nx,
                                   int ny, int nz, int nb, float* dw, int* err, cudaStream_t st) {
+  if (conv3_wgrad_fits(Cin, Cout))
+    return conv3_wgrad_tma(x, Cin, dy, Cout, 0, nx, ny, nz, nb, dw, err, st);
   Vol g{nx, ny, nz, nb};
   int V = nx * ny * nz * nb;
   int M = 27 * Cin;

@@ -53,6 +53,24 @@ cudaError_t conv3_tma(const __nv_bfloat16* x, int K, int nx, int ny, int nz, int
                       const __nv_bfloat16* mask, __nv_bfloat16* y_bf16, float* y_f32, int* err,
                       cudaStream_t st);
 
+// The driver's cuTensorMapEncodeTiled (PFN_cuTensorMapEncodeTiled_v12000), or
+// null.
+void* tensor_map_encoder();
+
+// Weight gradient with TMA-staged operands (k_wgrad.cu), accumulated into dw
+// (FP32): input channels in planes of 8 and output channels a multiple of 16;
+// pack 1: one output channel whose gradient gr is packed by conv3_pack_dx
+// with sign -1; pack 2: two input channels, x packed with sign +1.
+bool conv3_wgrad_fits(int Cin, int Cout);
+bool conv3_wgrad_packed_fits(int Cin, int Cout);
+cudaError_t conv3_wgrad_tma(const __nv_bfloat16* x, int Cin, const __nv_bfloat16* gr, int Cout,
+                            int pack, int nx, int ny, int nz, int nb, float* dw, int* err,
+                            cudaStream_t st);
+// The three x-shifts of a tensor of 1 or 2 channels as one plane of 8
+// channels: dst[u][j C + c] = src[u + sign (j - 1)][c], 0 outside the row.
+cudaError_t conv3_pack_dx(const __nv_bfloat16* src, int C, int nx, int ny, int nz, int nb,
+                          int sign, __nv_bfloat16* dst, cudaStream_t st);
+
 constexpr int NET_LAYERS = 9;
 struct NetLayer {
   int cin, cout, level, relu;
@@ -97,6 +115,7 @@ struct PyroNet {
   __nv_bfloat16* skip1() const {
     return c1.as<__nv_bfloat16>() + (size_t)8 * vol.half().voxels() * 8;
   }
+  pyro::DevBuf pk;  // packed x-shifts of the 1- and 2-channel tensors (backward)
   pyro::DevBuf g9, g8, gc0, g7, gc1, g6, g5, gp2, g4, g3, gp1, g2, g1;
   cudaStream_t stream = nullptr;
 

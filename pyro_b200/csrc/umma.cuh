@@ -116,6 +116,25 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* mbar, uint32_t parit
   return false;
 }
 
+// One lane of a converged warp, the same one every time.  Loops that issue
+// MMAs run warp-wide around it: descriptors computed by the whole warp live
+// in uniform registers, where the MMA reads them.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P1;\n\t"
+      "elect.sync _|P1, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, P1;\n\t"
+      "}"
+      : "=r"(p));
+  return p != 0;
+}
+// mbar_wait_bounded by a converged warp, the same answer in every lane.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* mbar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(mbar, parity)) != 0;
+}
+
 // Arm the barrier's phase with `bytes` of expected transactions (one
 // arrival).
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* mbar, uint32_t bytes) {

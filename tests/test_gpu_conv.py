@@ -101,3 +101,31 @@ def test_backward_data_and_weight(lib, Cin, Cout, dims):
                                         ptr(dw), None)
     assert rc == 0, lib.pyro_last_error()
     _close(dw, wr.grad.permute(0, 2, 3, 4, 1).reshape(Cout, 27, Cin))
+
+
+@pytest.mark.parametrize("Cin,Cout,dims,nb", [
+    (8, 16, (3, 5, 7), 1),       # one plane, a row shorter than a tile
+    (16, 16, (4, 9, 33), 2),     # a ragged tile in x and y, two volumes
+    (24, 48, (5, 8, 16), 1),     # three groups of output channels
+    (96, 32, (3, 6, 40), 2),     # two groups of input channels
+    (104, 16, (2, 3, 17), 1),    # a prime count of planes
+    (128, 128, (2, 4, 32), 1),   # the most channels
+    (64, 64, (1, 1, 1), 1),      # a single voxel
+    (16, 16, (40, 61, 70), 1),   # many tiles per CTA
+])
+def test_backward_weight_tma(lib, Cin, Cout, dims, nb):
+    """The TMA-staged weight gradient accumulates into dw; FP32 sums of exact
+    products in another order, as above."""
+    nz, ny, nx = dims
+    x, w, _ = _tensors(nb, Cin, nz, ny, nx, Cout, 4)
+    g = torch.Generator().manual_seed(5)
+    dy = torch.randn(nb, Cout, nz, ny, nx, generator=g).bfloat16().float().cuda()
+    wr = w.clone().requires_grad_(True)
+    Fn.conv3d(x, wr, None, padding=1).backward(dy)
+    ref = wr.grad.permute(0, 2, 3, 4, 1).reshape(Cout, 27, Cin)
+    dw = torch.full((Cout, 27, Cin), 0.5, dtype=torch.float32, device="cuda")
+    xc, dyc = _cl(x), _cl(dy)
+    rc = lib.pyro_conv3_backward_weight(ptr(xc), Cin, ptr(dyc), Cout, nx, ny, nz, nb,
+                                        ptr(dw), None)
+    assert rc == 0, lib.pyro_last_error()
+    _close(dw - 0.5, ref)
