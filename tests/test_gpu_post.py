@@ -70,3 +70,23 @@ def test_select_rejects_bad_arguments():
     assert lib.pyro_post_select(p, 4, 4, 16, p, p, p, ctypes.byref(v), None) == \
         _abi.PYRO_E_INVALID
     assert lib.pyro_post_develop(p, 4, 4, 1.0, 2.0, p, p, None, None) == _abi.PYRO_E_INVALID
+
+
+@pytest.mark.parametrize("h,w", [(1, 1), (5, 3), (3, 64), (33, 250), (122, 75), (61, 640),
+                                 (5, 4096),    # the widest rows in shared memory
+                                 (3, 17000)])  # past them: filters from global memory
+def test_glare_filters_bit_for_bit(h, w):
+    """The linear image after the glare mix, bit for bit the restatement's
+    running sums, for rows and columns shorter than a filter, ragged groups
+    of rows, and both forms of the filters."""
+    require_cuda()
+    dev = Developer(w, h)
+    cam = Camera(False, 0.0, 0.04)
+    lin_d = torch.empty(h * w * 3, dtype=torch.float32, device="cuda")
+    acc = _accum(h, w, h * 7 + w)
+    dev.develop(cam, torch.from_numpy(acc).cuda().data_ptr(), 1.0 / 30.0,
+                lin_out=lin_d.data_ptr())
+    lin = (acc[:, :3] / np.maximum(acc[:, 3:4], F32(1.0))).reshape(h, w, 3)
+    lin = lin * np.power(F32(2.0), cam.ev_offset)
+    lin = lin * (F32(1.0) - F32(0.04)) + glare(lin) * F32(0.04)
+    assert np.array_equal(lin_d.cpu().numpy().reshape(h, w, 3), lin)
