@@ -257,26 +257,16 @@ bool encode_planes(CUtensorMap* m, const bf16* p, int planes, int nx, int ny, in
          CUDA_SUCCESS;
 }
 
-// dst[u][j * C + c] = src[u + sign (j - 1)][c] for the three x-shifts j, 0
-// outside the row and in the channels past 3 C: a tensor of C <= 2 channels
-// as one plane of 8.
-template <int C>
-__global__ void __launch_bounds__(256) k_pack_dx(const bf16* __restrict__ src, size_t V, int nx,
-                                                 int sign, bf16* __restrict__ dst) {
+// dst[u][j] = src[u + sign (j - 1)] for the three x-shifts j, 0 outside the
+// row and in the channels past 3: a tensor of one channel as a plane of 8.
+__global__ void __launch_bounds__(256) k_pack_dx(const uint16_t* __restrict__ src, size_t V,
+                                                 int nx, int sign, uint4* __restrict__ dst) {
   const size_t u = blockIdx.x * (size_t)256 + threadIdx.x;
   if (u >= V) return;
   const int x = (int)((uint32_t)u % (uint32_t)nx);
-  __align__(16) bf16 o[8];
-#pragma unroll
-  for (int e = 0; e < 8; e++) o[e] = __float2bfloat16(0.0f);
-#pragma unroll
-  for (int j = 0; j < 3; j++) {
-    const int s = sign * (j - 1);
-    if ((unsigned)(x + s) >= (unsigned)nx) continue;
-#pragma unroll
-    for (int c = 0; c < C; c++) o[j * C + c] = src[(u + s) * C + c];
-  }
-  *reinterpret_cast<uint4*>(dst + u * 8) = *reinterpret_cast<const uint4*>(o);
+  const uint32_t lo = (unsigned)(x - sign) < (unsigned)nx ? src[u - sign] : 0u;
+  const uint32_t hi = (unsigned)(x + sign) < (unsigned)nx ? src[u + sign] : 0u;
+  dst[u] = make_uint4(lo | (uint32_t)src[u] << 16, hi, 0u, 0u);
 }
 
 }  // namespace
@@ -284,20 +274,12 @@ __global__ void __launch_bounds__(256) k_pack_dx(const bf16* __restrict__ src, s
 // Channel counts of the TMA form: planes of 8 input channels and pairs of
 // planes of output channels (N a multiple of 16).
 bool conv3_wgrad_fits(int Cin, int Cout) { return Cin % 8 == 0 && Cout % 16 == 0; }
-bool conv3_wgrad_packed_fits(int Cin, int Cout) {
-  return (Cin == 2 && Cout % 16 == 0) || (Cin % 8 == 0 && Cout == 1);
-}
 
-cudaError_t conv3_pack_dx(const bf16* src, int C, int nx, int ny, int nz, int nb, int sign,
-                          bf16* dst, cudaStream_t st) {
+cudaError_t conv3_pack_dx(const bf16* src, int nx, int ny, int nz, int nb, int sign, bf16* dst,
+                          cudaStream_t st) {
   const size_t V = (size_t)nx * ny * nz * nb;
-  const unsigned grid = (unsigned)((V + 255) / 256);
-  if (C == 1)
-    k_pack_dx<1><<<grid, 256, 0, st>>>(src, V, nx, sign, dst);
-  else if (C == 2)
-    k_pack_dx<2><<<grid, 256, 0, st>>>(src, V, nx, sign, dst);
-  else
-    return cudaErrorInvalidValue;
+  k_pack_dx<<<(unsigned)((V + 255) / 256), 256, 0, st>>>((const uint16_t*)src, V, nx, sign,
+                                                         (uint4*)dst);
   return cudaGetLastError();
 }
 

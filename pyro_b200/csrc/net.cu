@@ -118,16 +118,29 @@ __global__ void __launch_bounds__(NT) k_stats(const float* __restrict__ b,
   block_add(n, sc + SC_VOL + 2 * vol + 1);
 }
 
+// The network's input (b / s, solid) as one plane of 8 channels holding its
+// three x-shifts: channels 2 j + {0, 1} of voxel u are the values of voxel
+// u + j - 1, 0 outside the row, so that the first
+// layer and its weight gradient run on the tensor cores.
 __global__ void __launch_bounds__(NT) k_input(const float* __restrict__ b,
                                               const uint32_t* __restrict__ f, size_t cells,
-                                              int nb, const double* __restrict__ sc,
-                                              __nv_bfloat162* __restrict__ in0) {
+                                              int nx, int nb, const double* __restrict__ sc,
+                                              uint4* __restrict__ in0) {
   GRID_LOOP(i, cells * nb) {
-    int vol = (int)(i / cells);
-    double s = vol_rms(sc, vol);
-    bool solid = f[i] == 1u;
-    float v = (!solid && s > 0.0) ? (float)((double)b[i] / s) : 0.0f;
-    in0[i] = __floats2bfloat162_rn(v, solid ? 1.0f : 0.0f);
+    const int vol = (int)((uint32_t)i / (uint32_t)cells);
+    const int x = (int)((uint32_t)i % (uint32_t)nx);
+    const double s = vol_rms(sc, vol);
+    uint4 o = make_uint4(0, 0, 0, 0);
+    uint32_t* w = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      if ((unsigned)(x + j - 1) >= (unsigned)nx) continue;
+      const bool solid = f[i + j - 1] == 1u;
+      const float v = (!solid && s > 0.0) ? (float)((double)b[i + j - 1] / s) : 0.0f;
+      const __nv_bfloat162 h = __floats2bfloat162_rn(v, solid ? 1.0f : 0.0f);
+      w[j] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    in0[i] = o;
   }
 }
 
@@ -516,7 +529,7 @@ int PyroNet::ensure(NetVol v, bool bwd) {
     DevBuf* b;
     size_t n;
   };
-  std::vector<A> fw = {{&in0, V0 * 2},  {&e0a, V0 * 16}, {&p1, V1 * 16},
+  std::vector<A> fw = {{&in0, V0 * 8},  {&e0a, V0 * 16}, {&p1, V1 * 16},
                        {&e1a, V1 * 32}, {&p2, V2 * 32}, {&e2a, V2 * 64},
                        {&e2, V2 * 64},  {&c1, V1 * 96},  {&d1, V1 * 32}, {&c0, V0 * 48},
                        {&d0, V0 * 16}};
@@ -560,19 +573,13 @@ int PyroNet::forward(const float* b, const uint32_t* flags, NetVol v, cudaStream
   NET_CU(cudaMemsetAsync(scal.p, 0, scal.bytes, st));
   k_stats<<<dim3(std::min<unsigned>(blocks_for(cells), 148 * 4), v.nb), NT, 0, st>>>(b, flags,
                                                                                     cells, S);
-  k_input<<<blocks_for(cells * v.nb), NT, 0, st>>>(b, flags, cells, v.nb, S,
-                                                   in0.as<__nv_bfloat162>());
+  k_input<<<blocks_for(cells * v.nb), NT, 0, st>>>(b, flags, cells, v.nx, v.nb, S,
+                                                   in0.as<uint4>());
   NET_CU(cudaGetLastError());
   auto conv = [&](const bf16* x, int l, NetVol g, bf16* y, float* yf) -> cudaError_t {
     const NetLayer& L = NET_SPEC[l];
-    if (conv3_direct_fits(L.cin, L.cout))
-      return conv3_direct(x, L.cin, g.nx, g.ny, g.nz, g.nb, w(l), L.cout, bias(l), L.relu, y, yf,
-                          st);
-    if (L.cin % 16 == 0)
-      return conv3_tma(x, L.cin, g.nx, g.ny, g.nz, g.nb, wf(l), L.cout, bias(l), L.relu, nullptr,
-                       y, yf, E, st);
-    return conv3_forward(x, L.cin, g.nx, g.ny, g.nz, g.nb, w(l), L.cout, bias(l), L.relu, y, yf,
-                         E, st);
+    return conv3_tma(x, L.cin, L.cin % 16 ? 1 : 0, g.nx, g.ny, g.nz, g.nb, wf(l), L.cout, bias(l),
+                     L.relu, nullptr, y, yf, E, st);
   };
   auto B = [](const DevBuf& d) { return d.as<bf16>(); };
   // the skip connections e0, e1 are written straight into their planes of
@@ -623,17 +630,14 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
     const NetLayer& L = NET_SPEC[l];
     const bf16 *xs = x.as<bf16>(), *gs = dz.as<bf16>();
     cudaError_t e;
-    if (conv3_wgrad_packed_fits(L.cin, L.cout)) {  // the first and the last layer
-      const bool one = L.cout == 1;
-      e = conv3_pack_dx(one ? gs : xs, one ? 1 : L.cin, g.nx, g.ny, g.nz, g.nb, one ? -1 : 1,
-                        pk.as<bf16>(), st);
-      if (e != cudaSuccess) return e;
-      e = conv3_wgrad_tma(one ? xs : pk.as<bf16>(), L.cin, one ? pk.as<bf16>() : gs, L.cout,
-                          one ? 1 : 2, g.nx, g.ny, g.nz, g.nb, G + w_off[l], E, st);
-    } else {
+    if (L.cout == 1)  // the last layer: pk holds its gradient's shifts
+      e = conv3_wgrad_tma(xs, L.cin, pk.as<bf16>(), 1, 1, g.nx, g.ny, g.nz, g.nb, G + w_off[l], E,
+                          st);
+    else if (L.cin == 2)  // the first: in0 holds the input's
+      e = conv3_wgrad_tma(xs, 2, gs, L.cout, 2, g.nx, g.ny, g.nz, g.nb, G + w_off[l], E, st);
+    else
       e = conv3_backward_weight(xs, L.cin, gs, L.cout, g.nx, g.ny, g.nz, g.nb, G + w_off[l], E,
                                 st);
-    }
     if (e != cudaSuccess) return e;
     float* db = G + n_w + b_off[l];
     if (L.cout % 8 == 0)
@@ -646,12 +650,12 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
   };
   auto bd = [&](const DevBuf& dz, int l, NetVol g, const DevBuf* act, DevBuf& dx) -> cudaError_t {
     const NetLayer& L = NET_SPEC[l];
-    if (L.cout % 16 == 0)
-      return conv3_tma(dz.as<bf16>(), L.cout, g.nx, g.ny, g.nz, g.nb, wb(l), L.cin, nullptr, 0,
-                       act ? act->as<bf16>() : nullptr, dx.as<bf16>(), nullptr, E, st);
-    return conv3_backward_data(dz.as<bf16>(), L.cout, g.nx, g.ny, g.nz, g.nb, w(l), L.cin,
-                               act ? act->as<bf16>() : nullptr, dx.as<bf16>(), nullptr, E, st);
+    const bool one = L.cout == 1;
+    return conv3_tma(one ? pk.as<bf16>() : dz.as<bf16>(), L.cout, one ? -1 : 0, g.nx, g.ny, g.nz,
+                     g.nb, wb(l), L.cin, nullptr, 0, act ? act->as<bf16>() : nullptr,
+                     dx.as<bf16>(), nullptr, E, st);
   };
+  NET_CU(conv3_pack_dx(g9.as<bf16>(), v.nx, v.ny, v.nz, v.nb, -1, pk.as<bf16>(), st));
   NET_CU(wg(d0, g9, 8, v));
   NET_CU(bd(g9, 8, v, &d0, g8));
   NET_CU(wg(c0, g8, 7, v));

@@ -129,3 +129,37 @@ def test_backward_weight_tma(lib, Cin, Cout, dims, nb):
                                         ptr(dw), None)
     assert rc == 0, lib.pyro_last_error()
     _close(dw - 0.5, ref)
+
+
+@pytest.mark.parametrize("C,Cout,dims,nb", [
+    (16, 16, (1, 1, 1), 1),      # a single voxel
+    (16, 16, (5, 17, 9), 2),     # ragged in every direction, two volumes
+    (16, 16, (64, 160, 80), 1),  # four planes per tile, many tiles per CTA
+    (48, 16, (33, 70, 41), 1),   # the same with three channel groups
+    (16, 1, (70, 90, 60), 1),    # eight planes per tile, one column each
+    (16, 48, (21, 33, 40), 1),   # two planes per tile, wide columns
+    (64, 64, (3, 20, 30), 1),    # output channels split over CTAs
+    (128, 128, (2, 5, 11), 1),   # the most channels
+    (32, 24, (4, 18, 10), 1),    # 8-channel planes, not a multiple of 16
+    (16, 100, (2, 9, 8), 1),     # channels that fill no plane
+])
+def test_forward_tiles(lib, C, Cout, dims, nb):
+    """FP32 output against the reference as above; BF16 output, bit for bit the
+    same sums rounded."""
+    nz, ny, nx = dims
+    x, w, b = _tensors(nb, C, nz, ny, nx, Cout, 6)
+    ref = torch.relu(Fn.conv3d(x, w, b, padding=1))
+    xc, wk = _cl(x), _wk(w)
+    y32 = torch.full((nb, nz, ny, nx, Cout), 7.0, device="cuda")
+    y16 = torch.full((nb * nz * ny * nx * Cout,), 7.0, dtype=torch.bfloat16, device="cuda")
+    for y, f32 in ((y32, 1), (y16, 0)):
+        rc = lib.pyro_conv3_forward(ptr(xc), C, nx, ny, nz, nb, ptr(wk), Cout, ptr(b), 1, ptr(y),
+                                    f32, None)
+        assert rc == 0, lib.pyro_last_error()
+    got = y32.permute(0, 4, 1, 2, 3)
+    _close(got, ref)
+    if Cout % 8 == 0:
+        bf = y16.view(Cout // 8, nb, nz, ny, nx, 8).permute(1, 0, 5, 2, 3, 4).reshape(ref.shape)
+    else:
+        bf = y16.view(nb, nz, ny, nx, Cout).permute(0, 4, 1, 2, 3)
+    assert torch.equal(bf, got.bfloat16())
