@@ -109,142 +109,263 @@ __global__ void __launch_bounds__(256) k_mg_resid(Lvl d, float h2, const float* 
 
 // ------------------------------------------------------------ coarse solve
 // The coarsest level is swept 80 times per V-cycle (src/sim.rs:473), 160
-// dependent red-black passes over ~10-30 k cells.  One thread-block cluster
-// of up to 16 CTAs runs them all in a single launch: CTA r owns z-planes
-// [r*nz/C, (r+1)*nz/C) of phi in its shared memory, neighbours across a
-// slab boundary are read from the owning CTA's shared memory (distributed
-// shared memory), and the hardware cluster barrier separates the colour
-// passes.  Threads are sorted by colour: thread t holds, per colour c, the
-// cells q = t + T k (k < K) of the slab in the reference smoother's own
-// numbering (x = 2 hx + ((y + z + c) & 1), mg.wgsl:17-19), with the
-// neighbour mask, count and h^2 b in registers, so every lane of a warp
-// updates a cell of the pass's colour and a barrier waits on few warps.  A
-// thread loads all neighbours of its cells of the pass before it computes
-// any of them.  The arithmetic per cell is the reference's, in the same
-// order, so the result equals 160 separate passes bit for bit.
+// dependent red-black passes over ~1-30 k cells.  One thread-block cluster
+// runs them all in a single launch: CTA r owns z-planes [r nz / C,
+// (r + 1) nz / C) of phi in its shared memory, with a ghost plane on either
+// side.
+//
+// What bounds it is the latency of a pass, so a pass costs one block barrier
+// and one message to each neighbour: a thread that has updated a cell of the
+// slab's first or last plane stores it straight into the neighbour's ghost
+// plane with st.async, which also counts its bytes on the neighbour's
+// mbarrier, and the neighbour's threads wait for that count before they start
+// the next pass.  (Reading the neighbour's planes remotely between two
+// barriers of the whole cluster took 0.88 us a pass: a cluster barrier is
+// 0.24-0.32 us and a remote read 0.24.)
+// A ghost plane is not overwritten while it is read: a neighbour sends in
+// pass p + 1 only after it has all of this CTA's cells of pass p, and a thread
+// here sends a cell after it has loaded that cell's ghost neighbour; in pass
+// p + 1 itself this CTA reads the other colour of the ghosts.  The last pass sends nothing, so no store is in flight to a CTA
+// that ends.
+//
+// The two colours live in separate arrays, indexed by the reference
+// smoother's own numbering q = hx + hxn (y + ny z), x = 2 hx + ((y + z + c) &
+// 1) (mg.wgsl:17-19): the y and z neighbours of cell q are q +- hxn and
+// q +- hxn ny of the other colour, the x neighbours q and q - 1 or q + 1, so
+// loads and messages of a warp are contiguous.  Thread t holds cells t + T k
+// (k < K) of each colour, with the neighbours' addresses, the count and h^2 b
+// in registers.  The
+// arithmetic per cell is the reference's, in the same order, so the result
+// equals 160 separate passes bit for bit.
+// Measured, 80 sweeps: 20 x 40 x 20 144 -> 82 us, 16 x 30 x 16 113 -> 53 us,
+// 8 x 20 x 8 101 -> 43 us (0.16 us of a pass is one warp's chain of loads,
+// additions, division and barrier, 0.09 us the message).
 constexpr int COARSE_MAX_CLUSTER = 16;
 constexpr int COARSE_SMEM = 200 * 1024;
+// Threads per CTA at most with K cells per thread and colour (each keeps
+// ~22 K registers of cell state).
+constexpr int coarse_threads(int K) { return K == 1 ? 1024 : K == 2 ? 640 : 512; }
+constexpr uint32_t COARSE_SPINS = 1u << 22;
 
+// A cell of a thread: shared-memory addresses of its six neighbours (a place
+// that holds 0 where there is none to add: the sum starts at +0 and never
+// becomes -0, so adding +0 leaves its bits) and of itself.
 struct CoarseCell {
-  int j;             // index in the own slab (0 for an empty slot)
-  uint32_t meta;     // bits 0-5: fluid in-domain neighbour, bit 7: skip
-  float cnt;
-  float hb;
-  const float* zp;   // +z neighbour (local or remote); the cell itself when absent
-  const float* zm;   // -z neighbour
+  uint32_t nb[6], self;
+  float cnt, rcp, hb;
+  uint32_t to;  // bit 0: updated, bits 1 / 2: sent to the CTA below / above
 };
 
-template <typename TS, int T, int K>
-__global__ void __launch_bounds__(T, 1)
+__device__ __forceinline__ float lds(uint32_t a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts(uint32_t a, float v) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+// x / c for c = 1 .. 6 and rcp = 1 / c rounded: Markstein's correction of
+// x rcp (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990, theorem on division from a correctly rounded
+// reciprocal).  Equal to x / c bit for bit for 2^-100 <= |x| < 2^100 and for
+// x = +0 (every FP32 value checked against the division); other values take
+// the division.
+__device__ __forceinline__ float div_count(float x, float c, float rcp) {
+  const uint32_t u = __float_as_uint(x) & 0x7fffffffu;
+  if (u - 0x0d800000u < 0x64000000u || u == 0u) {
+    const float q = x * rcp;
+    return __fmaf_rn(__fmaf_rn(-q, c, x), rcp, q);
+  }
+  return x / c;
+}
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+// The shared::cluster address of this CTA's address `a` in CTA `rank`.
+__device__ __forceinline__ uint32_t map_rank(uint32_t a, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void send_async(uint32_t addr, float v, uint32_t mbar) {
+  asm volatile(
+      "st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr),
+      "r"(__float_as_uint(v)), "r"(mbar)
+      : "memory");
+}
+__device__ __forceinline__ bool wait_cluster(uint32_t mbar, uint32_t parity) {
+  for (uint32_t i = 0; i < COARSE_SPINS; i++) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred P1;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P1, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, P1;\n\t}"
+        : "=r"(ok)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
+template <typename TS, int K, bool SYM>
+__global__ void __launch_bounds__(coarse_threads(K), 1)
     k_mg_coarse_rb(Lvl d, float h2, const TS* __restrict__ b, const uint32_t* __restrict__ f,
-                   TS* __restrict__ p, int iters, float omega, int bc_mode, int symmetric) {
+                   TS* __restrict__ p, int iters, float omega, int bc_mode) {
   namespace cg = cooperative_groups;
   pdl_trigger();
   pdl_wait();
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ float sp[];
+  __shared__ __align__(8) uint64_t bar[2];
+  __shared__ float zero;
+  const int T = (int)blockDim.x;
   const int C = (int)cl.num_blocks();
   const int rank = (int)cl.block_rank();
-  const int plane = d.nx * d.ny;
-  const int z0 = rank * d.nz / C, z1 = (rank + 1) * d.nz / C;
-  const int own = (z1 - z0) * plane;
-  for (int j = threadIdx.x; j < own; j += T) sp[j] = ldv(p + z0 * plane + j);
-  cl.sync();  // every slab is loaded before any remote read
-  const int hxn = (d.nx + 1) / 2;
-  const int vpc = hxn * d.ny * (z1 - z0);  // virtual cells per colour
+  const int z0 = rank * d.nz / C, z1 = (rank + 1) * d.nz / C, planes = z1 - z0;
+  const int hxn = (d.nx + 1) / 2, pl = hxn * d.ny;
+  const int cap = ((d.nz + C - 1) / C + 2) * pl;  // floats of one colour, the same in every CTA
+  // sp[c cap + q]: colour c, plane 0 and plane planes + 1 are the ghosts
+  const int total = (planes + 2) * pl;
+  for (int q = threadIdx.x; q < total; q += T) {
+    const int hx = q % hxn, r = q / hxn, y = r % d.ny, z = z0 - 1 + r / d.ny;
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      const int x = 2 * hx + ((y + z + c) & 1);
+      sp[c * cap + q] = d.inb(x, y, z) ? ldv(p + d.idx(x, y, z)) : 0.0f;
+    }
+  }
+  const uint32_t bar0 = smem_addr(&bar[0]), sp0 = smem_addr(sp);
+  const uint32_t expect = 4u * (uint32_t)pl * (uint32_t)((rank > 0) + (rank + 1 < C));
+  if (threadIdx.x == 0) {
+    zero = 0.0f;
+    for (int i = 0; i < 2; i++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8u * i) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // what turns a cell's own address into its place at a neighbour: the ghost
+  // plane above the last plane of the CTA below, or the one below the first
+  // plane of the CTA above
+  uint32_t lo_off = 0, hi_off = 0, lo_bar = 0, hi_bar = 0;
+  if (rank > 0) {
+    const int below = z0 - (rank - 1) * d.nz / C;  // its planes
+    lo_off = map_rank(sp0, rank - 1) + 4u * (uint32_t)(below * pl) - sp0;
+    lo_bar = map_rank(bar0, rank - 1);
+  }
+  if (rank + 1 < C) {
+    hi_off = map_rank(sp0, rank + 1) - 4u * (uint32_t)(planes * pl) - sp0;
+    hi_bar = map_rank(bar0, rank + 1);
+  }
   CoarseCell cell[2][K];
 #pragma unroll
   for (int c = 0; c < 2; c++)
 #pragma unroll
     for (int k = 0; k < K; k++) {
-      CoarseCell& q = cell[c][k];
-      q.j = 0;
-      q.meta = 0x80u;
-      q.cnt = 1.0f;
-      q.hb = 0.0f;
-      q.zp = sp;
-      q.zm = sp;
+      CoarseCell& e = cell[c][k];
+      const uint32_t za = smem_addr(&zero);
+      e.self = za;
+#pragma unroll
+      for (int n = 0; n < 6; n++) e.nb[n] = za;
+      e.cnt = e.rcp = 1.0f;
+      e.hb = 0.0f;
+      e.to = 0u;
       const int v = threadIdx.x + T * k;
-      if (v >= vpc) continue;
+      if (v >= planes * pl) continue;
       const int hx = v % hxn, r = v / hxn;
       const int y = r % d.ny, zl = r / d.ny, z = z0 + zl;
-      const int x = 2 * hx + ((y + z + c) & 1);
+      const int par = (y + z + c) & 1, x = 2 * hx + par;
+      const uint32_t own = sp0 + 4u * (uint32_t)(c * cap + v + pl);
+      const uint32_t oth = sp0 + 4u * (uint32_t)((1 - c) * cap + v + pl);
+      e.self = own;
+      // every cell of a boundary plane is sent, updated or not: the number of
+      // bytes a CTA waits for does not depend on the flags
+      if (zl == 0 && rank > 0) e.to |= 2u;
+      if (zl == planes - 1 && rank + 1 < C) e.to |= 4u;
       if (x >= d.nx) continue;
-      const int rem = y * d.nx + x, j = zl * plane + rem;
       const int gi = d.idx(x, y, z);
-      q.j = j;
-      q.zp = sp + j;
-      q.zm = sp + j;
-      uint32_t meta = 0u;
+      const int step[6] = {par, par - 1, hxn, -hxn, pl, -pl};
       float cnt = 0.0f;
 #pragma unroll
-      for (int nb = 0; nb < 6; nb++) {
-        int ax = x + (nb == 0) - (nb == 1), ay = y + (nb == 2) - (nb == 3),
-            az = z + (nb == 4) - (nb == 5);
+      for (int n = 0; n < 6; n++) {
+        const int ax = x + (n == 0) - (n == 1), ay = y + (n == 2) - (n == 3),
+                  az = z + (n == 4) - (n == 5);
         if (ay < 0) continue;
         if (!d.inb(ax, ay, az)) {
           if (bc_mode == 0 || ay >= d.ny) cnt += 1.0f;
           continue;
         }
         if (f[d.idx(ax, ay, az)] == 1u) continue;
-        meta |= 1u << nb;
+        e.nb[n] = oth + 4u * (uint32_t)step[n];
         cnt += 1.0f;
-        if (nb >= 4) {
-          // owner of plane az and its slab-local index
-          int o = 0;
-          while (o + 1 < C && (o + 1) * d.nz / C <= az) o++;
-          const float* base = (az >= z0 && az < z1) ? sp : cl.map_shared_rank(sp, o);
-          const float* a = base + (az - o * d.nz / C) * plane + rem;
-          if (nb == 4) q.zp = a; else q.zm = a;
-        }
       }
-      if (f[gi] == 1u || cnt < 0.5f) meta |= 0x80u;
-      q.meta = meta;
-      q.cnt = cnt;
-      q.hb = h2 * ldv(b + gi);
+      if (f[gi] != 1u && cnt >= 0.5f) {
+        e.to |= 1u;
+        e.cnt = cnt;
+        e.rcp = 1.0f / cnt;
+      }
+      e.hb = h2 * ldv(b + gi);
     }
-  const int nx = d.nx;
+  cl.sync();  // the ghosts are loaded and every mbarrier is initialised
+  bool ok = true;
+  const int npass = 2 * iters;
+  // pass number `n` on colour c
+  auto pass = [&](const CoarseCell (&cells)[K], int n) {
+    const bool send = C > 1 && n + 1 < npass;
+    const uint32_t bo = 8u * (uint32_t)(n & 1);
+    // this pass's messages to this CTA are counted on bar[n & 1]
+    if (send && threadIdx.x == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar0 + bo),
+                   "r"(expect)
+                   : "memory");
+    // after a wait that ran out the passes go on without waiting
+    if (C > 1 && n > 0 && ok) ok = wait_cluster(bar0 + 8u - bo, (uint32_t)((n - 1) >> 1) & 1u);
+    float nbv[K][6], ownv[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+#pragma unroll
+      for (int j = 0; j < 6; j++) nbv[k][j] = lds(cells[k].nb[j]);
+      ownv[k] = lds(cells[k].self);
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const CoarseCell& e = cells[k];
+      float sum = 0.0f;
+#pragma unroll
+      for (int j = 0; j < 6; j++) sum += nbv[k][j];
+      float v = wmix(ownv[k], div_count(sum - e.hb, e.cnt, e.rcp), omega);
+      if (e.to & 1u) sts(e.self, v);
+      else v = ownv[k];
+      if (send) {
+        if (e.to & 2u) send_async(e.self + lo_off, v, lo_bar + bo);
+        if (e.to & 4u) send_async(e.self + hi_off, v, hi_bar + bo);
+      }
+    }
+    __syncthreads();
+  };
 #pragma unroll 1
   for (int it = 0; it < iters; it++) {
-    // symmetric: alternate red-black and black-red iterations (SSOR pairs)
-    const int first = symmetric ? (it & 1) : 0;
-#pragma unroll
-    for (int cc = 0; cc < 2; cc++) {
-      const int c = cc ^ first;
-      float nbv[K][6], ownv[K];
-      // every load of the pass first: absent neighbours read the cell itself
-      // (a valid address) and are not added
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        const CoarseCell& q = c ? cell[1][k] : cell[0][k];
-        const int j = q.j;
-        const uint32_t m = q.meta;
-        nbv[k][0] = sp[(m & 1u) ? j + 1 : j];
-        nbv[k][1] = sp[(m & 2u) ? j - 1 : j];
-        nbv[k][2] = sp[(m & 4u) ? j + nx : j];
-        nbv[k][3] = sp[(m & 8u) ? j - nx : j];
-        nbv[k][4] = *q.zp;
-        nbv[k][5] = *q.zm;
-        ownv[k] = sp[j];
-      }
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        const CoarseCell& q = c ? cell[1][k] : cell[0][k];
-        const uint32_t m = q.meta;
-        if (m & 0x80u) continue;
-        float sum = 0.0f;
-        if (m & 1u) sum += nbv[k][0];
-        if (m & 2u) sum += nbv[k][1];
-        if (m & 4u) sum += nbv[k][2];
-        if (m & 8u) sum += nbv[k][3];
-        if (m & 16u) sum += nbv[k][4];
-        if (m & 32u) sum += nbv[k][5];
-        sp[q.j] = wmix(ownv[k], (sum - q.hb) / q.cnt, omega);
-      }
-      cl.sync();
+    if (SYM && (it & 1)) {  // alternate red-black and black-red iterations
+      pass(cell[1], 2 * it);
+      pass(cell[0], 2 * it + 1);
+    } else {
+      pass(cell[0], 2 * it);
+      pass(cell[1], 2 * it + 1);
     }
   }
-  for (int j = threadIdx.x; j < own; j += T) stv(p + z0 * plane + j, sp[j]);
+  // A wait that ran out: the level becomes NaN, which the residual statistics
+  // and the solvers' convergence test report.
+  const bool all_ok = __syncthreads_and(ok) != 0;
+  for (int v = threadIdx.x; v < planes * pl; v += T) {
+    const int hx = v % hxn, r = v / hxn, y = r % d.ny, z = z0 + r / d.ny;
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      const int x = 2 * hx + ((y + z + c) & 1);
+      if (x < d.nx)
+        stv(p + d.idx(x, y, z), all_ok ? sp[c * cap + v + pl] : __int_as_float(0x7fc00000));
+    }
+  }
+  cl.sync();  // no CTA ends while another may still send to it
 }
 
 __global__ void k_f32_to_bf16(const float* __restrict__ a, __nv_bfloat16* __restrict__ b,
@@ -262,60 +383,53 @@ __global__ void k_bf16_to_f32(const __nv_bfloat16* __restrict__ a, float* __rest
   if (i < n) b[i] = __bfloat162float(a[i]);
 }
 
-// Threads per CTA and cells per thread and colour of the coarse kernel, in
-// the order tried: the first whose T * K covers a CTA's cells of one colour.
-// Measured on the 2 cm pool's 20 x 40 x 20 level (16 CTAs, 800 cells of a
-// colour per CTA, 80 sweeps): 512 threads x 2 cells 142 us, 256 x 4 154 us,
-// 128 x 8 229 us -- the barrier and the remote loads of a pass set its
-// length, and fewer warps hide less of it.
-struct CoarseShape {
-  int T, K;
-};
-constexpr CoarseShape COARSE_SHAPES[] = {{512, 2}, {512, 4}, {256, 8}};
+// Shared memory of a CTA: two colours of its planes and two ghost planes.
+size_t coarse_smem(Dims3 d, int C) {
+  return (size_t)((d.nz + C - 1) / C + 2) * ((d.nx + 1) / 2) * d.ny * 2 * 4;
+}
 
-// Cluster size and shape for a level: the largest cluster of 16 / 8 whose
-// slabs fit a shape and the shared memory; {0, 0} when none does.
+// Cluster size, cells per thread and colour and threads per CTA for a level;
+// C = 0 when none fits.  The largest cluster: a message to a neighbour costs
+// less than the warps that more planes per CTA would add (20 x 30 x 20: 67 us
+// on 16 CTAs, 89 on 8; 8 x 20 x 8: 43 us on 8, 44 on 4).  As few
+// cells per thread as fit: the same cells in fewer warps wait longer (two per
+// thread instead of one: 20 x 40 x 20 88 us against 82, 16 x 30 x 16 65
+// against 53).
 struct CoarsePlan {
-  int C = 0;
-  CoarseShape s{0, 0};
+  int C = 0, K = 0, T = 0;
 };
 CoarsePlan coarse_plan(Dims3 d, int max_cluster) {
   CoarsePlan pl;
-  if (d.nz < 1) return pl;
-  for (int C : {COARSE_MAX_CLUSTER, 8}) {
-    if (C > max_cluster) continue;
+  for (int C : {COARSE_MAX_CLUSTER, 8, 4, 2}) {
+    if (C > max_cluster || C > d.nz) continue;
     const int planes = (d.nz + C - 1) / C;
-    const size_t vpc = (size_t)((d.nx + 1) / 2) * d.ny * planes;
-    if ((size_t)planes * d.nx * d.ny * 4 > (size_t)COARSE_SMEM) continue;
-    for (const CoarseShape& s : COARSE_SHAPES)
-      if ((size_t)s.T * s.K >= vpc) {
-        pl.C = C;
-        pl.s = s;
-        return pl;
-      }
+    const int vpc = (d.nx + 1) / 2 * d.ny * planes;
+    if (coarse_smem(d, C) > (size_t)COARSE_SMEM) continue;
+    for (int K : {1, 2, 4}) {
+      const int T = ((vpc + K - 1) / K + 31) / 32 * 32;
+      if (T > coarse_threads(K)) continue;
+      pl.C = C;
+      pl.K = K;
+      pl.T = T;
+      return pl;
+    }
   }
   return pl;
 }
 
-template <typename TS, int T, int K>
+template <typename TS, int K, bool SYM>
 cudaError_t coarse_launch(const CoarsePlan& pl, Dims3 d, float h, const TS* b, const uint32_t* f,
-                          TS* p, int iters, float omega, int bc_mode, cudaStream_t st,
-                          int symmetric) {
-  auto kern = k_mg_coarse_rb<TS, T, K>;
-  static bool attr = false;  // attributes are per function, set once
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         COARSE_SMEM);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
-  const size_t smem = (size_t)((d.nz + pl.C - 1) / pl.C) * d.nx * d.ny * 4;
+                          TS* p, int iters, float omega, int bc_mode, cudaStream_t st) {
+  auto kern = k_mg_coarse_rb<TS, K, SYM>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       COARSE_SMEM);
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)pl.C, 1, 1);
-  cfg.blockDim = dim3((unsigned)T, 1, 1);
-  cfg.dynamicSmemBytes = smem;
+  cfg.blockDim = dim3((unsigned)pl.T, 1, 1);
+  cfg.dynamicSmemBytes = coarse_smem(d, pl.C);
   cfg.stream = st;
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -327,7 +441,7 @@ cudaError_t coarse_launch(const CoarsePlan& pl, Dims3 d, float h, const TS* b, c
   cfg.attrs = at;
   cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kern, Lvl{d.nx, d.ny, d.nz}, h * h, b, f, p, iters, omega,
-                            bc_mode, symmetric);
+                            bc_mode);
 }
 
 // The largest cluster this device co-schedules for the coarse kernel (16
@@ -335,7 +449,7 @@ cudaError_t coarse_launch(const CoarsePlan& pl, Dims3 d, float h, const TS* b, c
 int coarse_max_cluster() {
   static int mc = 0;
   if (mc) return mc;
-  auto kern = k_mg_coarse_rb<float, 256, 8>;
+  auto kern = k_mg_coarse_rb<float, 2, false>;
   int q = 8;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
           cudaSuccess &&
@@ -343,7 +457,7 @@ int coarse_max_cluster() {
           cudaSuccess) {
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3(COARSE_MAX_CLUSTER, 1, 1);
-    c.blockDim = dim3(256, 1, 1);
+    c.blockDim = dim3(coarse_threads(2), 1, 1);
     c.dynamicSmemBytes = 64 * 1024;
     if (cudaOccupancyMaxPotentialClusterSize(&q, kern, &c) != cudaSuccess) q = 8;
   }
@@ -358,11 +472,18 @@ cudaError_t mg_coarse_t(Dims3 d, float h, const TS* b, const uint32_t* f, TS* p,
                         float omega, int bc_mode, cudaStream_t st, int symmetric = 0) {
   const CoarsePlan pl = coarse_plan(d, coarse_max_cluster());
   if (pl.C == 0) return cudaErrorInvalidValue;
-  if (pl.s.K == 2)
-    return coarse_launch<TS, 512, 2>(pl, d, h, b, f, p, iters, omega, bc_mode, st, symmetric);
-  if (pl.s.K == 4)
-    return coarse_launch<TS, 512, 4>(pl, d, h, b, f, p, iters, omega, bc_mode, st, symmetric);
-  return coarse_launch<TS, 256, 8>(pl, d, h, b, f, p, iters, omega, bc_mode, st, symmetric);
+#define PYRO_COARSE(K)                                                                          \
+  case K:                                                                                      \
+    return symmetric                                                                           \
+               ? coarse_launch<TS, K, true>(pl, d, h, b, f, p, iters, omega, bc_mode, st)      \
+               : coarse_launch<TS, K, false>(pl, d, h, b, f, p, iters, omega, bc_mode, st)
+  switch (pl.K) {
+    PYRO_COARSE(1);
+    PYRO_COARSE(2);
+    PYRO_COARSE(4);
+    default: return cudaErrorInvalidValue;
+  }
+#undef PYRO_COARSE
 }
 
 }  // namespace

@@ -397,6 +397,30 @@ def test_mg_coarse_solve_equals_80_sor_sweeps(lib, nx, ny, nz, seed, h):
     assert np.array_equal(host(pd), e)
 
 
+@pytest.mark.parametrize("nx,ny,nz,seed,h", [
+    (2, 3, 2, 21, 0.3),      # two CTAs, the smallest level
+    (7, 11, 5, 22, 0.3),     # four CTAs, odd rows
+    (40, 50, 16, 23, 0.16),  # 1,000 cells of a colour per CTA: one per thread
+    (31, 40, 32, 24, 0.16),  # 1,280: two per thread
+    (51, 38, 31, 25, 0.16),  # 1,976: four per thread
+    (64, 64, 40, 26, 0.16),  # more than a cluster holds: one launch per pass
+])
+def test_mg_coarse_solve_cluster_shapes(lib, nx, ny, nz, seed, h):
+    """Every cluster size and thread shape of the coarse kernel, and the passes
+    that take over where none fits, bit for bit the oracle's sweeps."""
+    rng = np.random.default_rng(seed)
+    f = (rng.random((nz, ny, nx)) < 0.15).astype(np.uint32)
+    b = rng.normal(0, 1, (nz, ny, nx)).astype(np.float32)
+    p = rng.normal(0, 0.1, (nz, ny, nx)).astype(np.float32)
+    pd, bd, fd = dev(p), dev(b), dev(f)
+    assert lib.pyro_k_mg_coarse(nx, ny, nz, h, ptr(bd), ptr(fd), ptr(pd), 12, 1.6, None) == 0
+    e = p
+    for _ in range(12):
+        for c in (0, 1):
+            e = oracle.mg_smooth((nx, ny, nz), h, b, f, e, c, 1.6)
+    assert np.array_equal(host(pd), e)
+
+
 @pytest.mark.parametrize("nx,ny,nz,seed,h", [(20, 40, 20, 8, 0.16), (32, 32, 22, 9, 0.2),
                                              (8, 20, 8, 10, 0.32)])
 @pytest.mark.parametrize("bc_mode", [0, 1])
