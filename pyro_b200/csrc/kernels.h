@@ -72,6 +72,9 @@ cudaError_t launch_render_cdf(long n, const float* ecell, float* cdf, void* scra
 // The volume path tracer (k_trace.cu) on the packed volumes: camera rays
 // into accum, the two light caches, and the caches' separable blur (radius
 // 1 .. render_blur_max_radius()).
+// Gives back the memory that the renderer's scratch pool keeps on the current
+// device.
+void ray_pool_trim();
 cudaError_t launch_render_trace(const PyroRenderParams& R, const void* vol, const void* sol,
                                 const void* vel, const float* bricks, const float* lut,
                                 const float* ecdf, const void* lvA, const void* lvB, int lx,

@@ -17,6 +17,11 @@ int DevBuf::alloc(size_t n) {
   release();
   if (n == 0) return PYRO_OK;
   cudaError_t e = cudaMalloc(&p, n);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    ray_pool_trim();
+    e = cudaMalloc(&p, n);
+  }
   if (e != cudaSuccess) {
     p = nullptr;
     set_error(std::string("cudaMalloc(") + std::to_string(n) + "): " + cudaGetErrorString(e));

@@ -206,6 +206,35 @@ def _glowing_frame(nx, ny, nz, seed):
     return P, d
 
 
+@pytest.mark.parametrize("dims,emit", [((16, 16, 16), "all"),    # the CDF's steps are bucket edges
+                                       ((16, 16, 16), "first"),  # one emitting cell
+                                       ((16, 16, 16), "last"),
+                                       ((9, 21, 5), "some")])    # fewer cells than buckets
+def test_light_caches_pick_cells_as_the_oracle(lib, dims, emit):
+    """The caches' rays find their emitting cells through the guide to the
+    CDF; against the oracle's plain search, the tolerances of the frame test."""
+    nx, ny, nz = dims
+    P, d = _glowing_frame(nx, ny, nz, seed=3)
+    e = np.zeros((nz, ny, nx), np.float32)
+    if emit == "all":
+        e[...] = 1.0
+    elif emit == "some":
+        e[...] = np.random.default_rng(5).random(e.shape) < 0.05
+    else:
+        e.reshape(-1)[0 if emit == "first" else -1] = 2.0
+    d["ecdf"] = oracle.render_cdf(e)
+    rows = _rp_rows(P, 8, 8, 1, 3, True)
+    rp = _abi.PyroRenderParams.from_rows(rows)
+    lvd = ((nx + 1) // 2, (ny + 1) // 2, (nz + 1) // 2)
+    a, bb = _half_empty((*lvd[::-1], 4)), _half_empty((*lvd[::-1], 4))
+    b = _bind(d)
+    render.lightvol(rp, *_args(b), lvd, a, bb, rays=12)
+    ea, eb = oracle.render_lightvol(rows, d["vol"], d["solt"], d["vel"], d["bricks"], d["lut"],
+                                    d["ecdf"], lvd, lv_n=12)
+    _cache_close(host(a), ea, max_bad=5e-3)
+    _cache_close(host(bb), eb, max_bad=5e-3)
+
+
 @pytest.mark.parametrize("mode", ["cache", "path"])
 def test_frame_vs_oracle(lib, mode):
     """A whole frame on a 24 x 40 x 20 grid: caches (16 rays), blur chain and
