@@ -24,6 +24,9 @@ struct ConvEpi {
   const float* bias;
   const bf16* mask;
   int V, Nout, relu;
+  // up != 0: out_bf16 is over a volume of twice the size (fx, fy, fz; fV voxels
+  // in all), and a voxel's result goes to its children there (k_conv3.cu)
+  int up, fx, fy, fz, fV;
   __device__ void operator()(int m, int col, const float (&v)[16]) const {
     if (m < 0 || m >= V) return;
     if (out_bf16 && (Nout & 15) == 0) {

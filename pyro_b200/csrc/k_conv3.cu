@@ -41,9 +41,10 @@
 // shifted copies of x; 2 -> 16 and 16 -> 1 channels on the CUDA cores), in us:
 // 2 -> 16 405 -> 101, 16 -> 16 773 -> 244, 48 -> 16 1990 -> 598, 16 -> 1 493
 // -> 159; on 80 x 160 x 80, 96 -> 32 522 -> 320; the data gradient 16 -> 48 on
-// two 128^3 volumes 1411 -> 370.  What bounds it now: the loads, 16 cycles per
-// 160-byte row of a box whatever the boxes' number, 216 rows for the 54 MMAs
-// (2592 cycles) of a stage of four planes.
+// two 128^3 volumes 1411 -> 370.  What bounds it now: the MMAs' issue
+// (48 -> 16: 54 MMAs of 48 cycles per 512 voxels and group are 0.44 ms at
+// 1.9 GHz; copying the input with cp.async from four warps measured 684 us
+// against 598 with the boxes).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -332,7 +333,21 @@ __global__ void __launch_bounds__(C3_THREADS, 1)
                   uw[e] &= (lo > 0.0f ? 0x0000FFFFu : 0u) | (hi > 0.0f ? 0xFFFF0000u : 0u);
                 }
               }
-              reinterpret_cast<uint4*>(ep.out_bf16)[o[k] + (size_t)h * ep.V] = u;
+              if (ep.up) {
+                const int z = 2 * (z0 + (ZO == 1 ? 0 : (k0 + k) / gpz));
+                uint4* q8 = reinterpret_cast<uint4*>(ep.out_bf16) +
+                            (size_t)(((co0 + c[k]) >> 3) + h) * ep.fV;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                  const int fz = z + (j >> 1), fy = 2 * y + (j & 1);
+                  if (fz >= ep.fz || fy >= ep.fy) continue;
+                  uint4* row = q8 + (((size_t)tib * ep.fz + fz) * ep.fy + fy) * ep.fx + 2 * x;
+                  row[0] = u;
+                  if (2 * x + 1 < ep.fx) row[1] = u;
+                }
+              } else {
+                reinterpret_cast<uint4*>(ep.out_bf16)[o[k] + (size_t)h * ep.V] = u;
+              }
             }
           }
         }
@@ -432,7 +447,8 @@ C3Plan c3_plan(int nx, int ny, int nz, int nb, int groups, int N_out, bool pack,
 // N <= 128 output channels.  x must be 16-byte aligned.
 cudaError_t conv3_tma(const bf16* x, int K, int pack, int nx, int ny, int nz, int nb,
                       const bf16* w_tap, int N, const float* bias, int relu, const bf16* mask,
-                      bf16* y_bf16, float* y_f32, int* err, cudaStream_t st) {
+                      bf16* y_bf16, float* y_f32, int* err, cudaStream_t st, const NetVol* fine) {
+  if (fine && (!y_bf16 || N % 16)) return cudaErrorInvalidValue;
   if ((pack ? K < 1 || K > 2 : K % 16 != 0) || N < 1 || N > C3_MAX_CO)
     return cudaErrorInvalidValue;
   PFN_cuTensorMapEncodeTiled_v12000 enc = (PFN_cuTensorMapEncodeTiled_v12000)tensor_map_encoder();
@@ -483,7 +499,9 @@ cudaError_t conv3_tma(const bf16* x, int K, int pack, int nx, int ny, int nz, in
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return e;
-  ConvEpi ep{y_bf16, y_f32, bias, mask, nx * ny * nz * nb, N, relu};
+  ConvEpi ep{y_bf16, y_f32, bias, mask, nx * ny * nz * nb, N, relu,
+             fine ? 1 : 0, fine ? fine->nx : 0, fine ? fine->ny : 0, fine ? fine->nz : 0,
+             fine ? (int)fine->voxels() : 0};
   const int ctas = std::max(1, std::min(g.ntiles, nsm / pl.split));
   kern<<<dim3((unsigned)ctas, (unsigned)pl.split), C3_THREADS, smem, st>>>(tx, w_tap, g, ep, err);
   return cudaGetLastError();

@@ -27,6 +27,15 @@
 
 namespace pyro {
 
+struct NetVol {
+  int nx, ny, nz, nb;
+  size_t voxels() const { return (size_t)nx * ny * nz * nb; }
+  NetVol half() const { return NetVol{(nx + 1) / 2, (ny + 1) / 2, (nz + 1) / 2, nb}; }
+  bool operator==(const NetVol& o) const {
+    return nx == o.nx && ny == o.ny && nz == o.nz && nb == o.nb;
+  }
+};
+
 cudaError_t conv3_forward(const __nv_bfloat16* x, int C, int nx, int ny, int nz, int nb,
                           const __nv_bfloat16* w, int Cout, const float* bias, int relu,
                           __nv_bfloat16* y_bf16, float* y_f32, int* err, cudaStream_t st);
@@ -47,13 +56,15 @@ cudaError_t conv3_direct(const __nv_bfloat16* x, int C, int nx, int ny, int nz, 
 // TMA-staged convolution (k_conv3.cu) on tap-major weights prepared by
 // conv3_prep_weights: input channels K a multiple of 16, or (pack = +-1) the
 // K = 1 or 2 channels of a tensor whose x-shifts are packed into one plane of
-// 8 channels, channel j K + k holding voxel u + pack (j - 1).
+// 8 channels, channel j K + k holding voxel u + pack (j - 1).  fine (BF16
+// output of a multiple of 16 channels): every voxel's result is written to its
+// children in the first planes of a tensor over that volume, y_bf16.
 cudaError_t conv3_prep_weights(const __nv_bfloat16* w, int Cout, int Cin, int backward,
                                __nv_bfloat16* w_tap, cudaStream_t st);
 cudaError_t conv3_tma(const __nv_bfloat16* x, int K, int pack, int nx, int ny, int nz, int nb,
                       const __nv_bfloat16* w_tap, int N, const float* bias, int relu,
                       const __nv_bfloat16* mask, __nv_bfloat16* y_bf16, float* y_f32, int* err,
-                      cudaStream_t st);
+                      cudaStream_t st, const NetVol* fine = nullptr);
 
 // The driver's cuTensorMapEncodeTiled (PFN_cuTensorMapEncodeTiled_v12000), or
 // null.
@@ -81,15 +92,6 @@ constexpr NetLayer NET_SPEC[NET_LAYERS] = {{2, 16, 0, 1},  {16, 16, 0, 1}, {16, 
                                            {32, 32, 1, 1}, {32, 64, 2, 1}, {64, 64, 2, 1},
                                            {96, 32, 1, 1}, {48, 16, 0, 1}, {16, 1, 0, 0}};
 
-struct NetVol {
-  int nx, ny, nz, nb;
-  size_t voxels() const { return (size_t)nx * ny * nz * nb; }
-  NetVol half() const { return NetVol{(nx + 1) / 2, (ny + 1) / 2, (nz + 1) / 2, nb}; }
-  bool operator==(const NetVol& o) const {
-    return nx == o.nx && ny == o.ny && nz == o.nz && nb == o.nb;
-  }
-};
-
 }  // namespace pyro
 
 // Parameters: all weights first ([Cout][27][Cin] per layer, layers in
@@ -109,7 +111,7 @@ struct PyroNet {
   // activation buffers for the current volume shape
   pyro::NetVol vol{0, 0, 0, 0};
   bool has_bwd = false;
-  pyro::DevBuf in0, e0a, p1, e1a, p2, e2a, e2, c1, d1, c0, d0, out, res;
+  pyro::DevBuf in0, e0a, p1, e1a, p2, e2a, c1, c0, d0, out, res;
   // skip activations e0 (16 channels, level 0) and e1 (32, level 1): the
   // last 2 / 4 planes of the concatenations c0 / c1
   __nv_bfloat16* skip0() const { return c0.as<__nv_bfloat16>() + (size_t)4 * vol.voxels() * 8; }
