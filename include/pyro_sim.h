@@ -198,7 +198,8 @@ int pyro_sim_profile_step(PyroSim* sim, float dt, float time, float ign_on,
  * 0 level masks and coarse flags, 1 level-0 colour pass, 2 level-0
  * restriction, 3 prolongation onto level 0, 4 colour pass on a middle
  * level, 5 restriction from a middle level, 6 prolongation onto a middle
- * level, 7 the coarsest-level solve.  No counterpart in the reference. */
+ * level, 7 the coarsest-level solve; a launch of several passes counts as
+ * that many.  No counterpart in the reference. */
 #define PYRO_PROFILE_MG_CLASSES 8
 int pyro_sim_profile_pressure(PyroSim* sim, float* ms_out, int* launches_out,
                               int n);
@@ -408,6 +409,14 @@ int pyro_k_mg_flags_down(uint32_t fnx, uint32_t fny, uint32_t fnz,
 int pyro_k_mg_pass(uint32_t nx, uint32_t ny, uint32_t nz, float h,
                    const void* b, const uint8_t* meta, void* phi, int color,
                    float omega, int bc_mode, int storage, void* stream);
+/* `sweeps` smoother sweeps, both colours each (colour 1 first when black_first
+ * != 0), as one launch: equal to 2 sweeps pyro_k_mg_pass calls bit for bit.
+ * For levels that fit a thread-block cluster with one cell of a colour per
+ * thread, as the V-cycle runs them there; PYRO_E_INVALID for others. */
+int pyro_k_mg_sweeps(uint32_t nx, uint32_t ny, uint32_t nz, float h,
+                     const void* b, const uint8_t* meta, void* phi, int sweeps,
+                     float omega, int black_first, int bc_mode, int storage,
+                     void* stream);
 int pyro_k_mg_restrict_m(uint32_t fnx, uint32_t fny, uint32_t fnz, float fh,
                          const void* pf, const void* bf, const uint8_t* mf,
                          uint32_t cnx, uint32_t cny, uint32_t cnz, void* bc,

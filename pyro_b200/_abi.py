@@ -215,6 +215,7 @@ SIGNATURES = {
     "pyro_k_mg_meta": [_U32, _U32, _U32, _P, _P, _P],
     "pyro_k_mg_flags_down": [_U32, _U32, _U32, _P, _U32, _U32, _U32, _P, _P],
     "pyro_k_mg_pass": [_U32, _U32, _U32, _F, _P, _P, _P, _I, _F, _I, _I, _P],
+    "pyro_k_mg_sweeps": [_U32, _U32, _U32, _F, _P, _P, _P, _I, _F, _I, _I, _I, _P],
     "pyro_k_mg_restrict_sym": [_U32, _U32, _U32, _F, _P, _P, _P, _U32, _U32, _U32, _P, _P, _P,
                                _I, _I, _P],
     "pyro_k_mg_pass_first": [_U32, _U32, _U32, _F, _P, _P, _P, _P, _I, _F, _I, _I, _P],

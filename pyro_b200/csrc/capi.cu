@@ -258,6 +258,23 @@ int pyro_k_mg_pass(uint32_t nx, uint32_t ny, uint32_t nz, float h, const void* b
              "pyro_k_mg_pass");
 }
 
+int pyro_k_mg_sweeps(uint32_t nx, uint32_t ny, uint32_t nz, float h, const void* b,
+                     const uint8_t* meta, void* phi, int sweeps, float omega, int black_first,
+                     int bc_mode, int storage, void* stream) {
+  clear_error();
+  PYRO_REQUIRE(dims_ok(nx, ny, nz), "pyro_k_mg_sweeps: invalid grid dimensions");
+  PYRO_REQUIRE(b && meta && phi, "pyro_k_mg_sweeps: null buffer");
+  PYRO_REQUIRE(sweeps >= 0, "pyro_k_mg_sweeps: sweeps must be >= 0");
+  PYRO_REQUIRE(bc_mode == 0 || bc_mode == 1, "pyro_k_mg_sweeps: bc_mode must be 0 or 1");
+  PYRO_REQUIRE(storage == PYRO_MG_F32 || storage == PYRO_MG_BF16,
+               "pyro_k_mg_sweeps: storage must be PYRO_MG_F32 or PYRO_MG_BF16");
+  Dims3 d{(int)nx, (int)ny, (int)nz};
+  PYRO_REQUIRE(mg_sweeps_fit(d), "pyro_k_mg_sweeps: the level does not fit a cluster");
+  return ret(launch_mg_sweeps(d, h, b, meta, phi, sweeps, omega, black_first != 0, bc_mode,
+                              storage == PYRO_MG_BF16, S(stream)),
+             "pyro_k_mg_sweeps");
+}
+
 int pyro_k_mg_pass_first(uint32_t nx, uint32_t ny, uint32_t nz, float h, const float* r,
                          void* bq, const uint8_t* meta, void* phi, int color, float omega,
                          int bc_mode, int storage, void* stream) {

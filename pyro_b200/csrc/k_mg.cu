@@ -209,10 +209,17 @@ __device__ __forceinline__ bool wait_cluster(uint32_t mbar, uint32_t parity) {
   return false;
 }
 
-template <typename TS, int K, bool SYM>
+// ORDER of an iteration's colours: red-black, black-red, or the two in turn.
+// SMOOTH: the sweeps of a smoother: neighbours from the level's masks (`meta`
+// instead of the flags), and a cell's value is rounded to the storage type
+// after every pass, as separate pass launches store it.
+enum SweepOrder { RED_BLACK, BLACK_RED, ALTERNATE };
+
+template <typename TS, int K, int ORDER, bool SMOOTH>
 __global__ void __launch_bounds__(coarse_threads(K), 1)
     k_mg_coarse_rb(Lvl d, float h2, const TS* __restrict__ b, const uint32_t* __restrict__ f,
-                   TS* __restrict__ p, int iters, float omega, int bc_mode) {
+                   const uint8_t* __restrict__ meta, TS* __restrict__ p, int iters, float omega,
+                   int bc_mode) {
   namespace cg = cooperative_groups;
   pdl_trigger();
   pdl_wait();
@@ -286,6 +293,7 @@ __global__ void __launch_bounds__(coarse_threads(K), 1)
       const int gi = d.idx(x, y, z);
       const int step[6] = {par, par - 1, hxn, -hxn, pl, -pl};
       float cnt = 0.0f;
+      const uint32_t m = SMOOTH ? meta[gi] : 0u;  // bits 0-5: fluid neighbours, 6: solid
 #pragma unroll
       for (int n = 0; n < 6; n++) {
         const int ax = x + (n == 0) - (n == 1), ay = y + (n == 2) - (n == 3),
@@ -295,11 +303,11 @@ __global__ void __launch_bounds__(coarse_threads(K), 1)
           if (bc_mode == 0 || ay >= d.ny) cnt += 1.0f;
           continue;
         }
-        if (f[d.idx(ax, ay, az)] == 1u) continue;
+        if (SMOOTH ? !((m >> n) & 1u) : f[d.idx(ax, ay, az)] == 1u) continue;
         e.nb[n] = oth + 4u * (uint32_t)step[n];
         cnt += 1.0f;
       }
-      if (f[gi] != 1u && cnt >= 0.5f) {
+      if (!(SMOOTH ? (m & 0x40u) != 0u : f[gi] == 1u) && cnt >= 0.5f) {
         e.to |= 1u;
         e.cnt = cnt;
         e.rcp = 1.0f / cnt;
@@ -334,6 +342,7 @@ __global__ void __launch_bounds__(coarse_threads(K), 1)
 #pragma unroll
       for (int j = 0; j < 6; j++) sum += nbv[k][j];
       float v = wmix(ownv[k], div_count(sum - e.hb, e.cnt, e.rcp), omega);
+      if (SMOOTH && sizeof(TS) == 2) v = __bfloat162float(__float2bfloat16_rn(v));
       if (e.to & 1u) sts(e.self, v);
       else v = ownv[k];
       if (send) {
@@ -345,7 +354,7 @@ __global__ void __launch_bounds__(coarse_threads(K), 1)
   };
 #pragma unroll 1
   for (int it = 0; it < iters; it++) {
-    if (SYM && (it & 1)) {  // alternate red-black and black-red iterations
+    if (ORDER == BLACK_RED || (ORDER == ALTERNATE && (it & 1))) {
       pass(cell[1], 2 * it);
       pass(cell[0], 2 * it + 1);
     } else {
@@ -417,10 +426,11 @@ CoarsePlan coarse_plan(Dims3 d, int max_cluster) {
   return pl;
 }
 
-template <typename TS, int K, bool SYM>
+template <typename TS, int K, int ORDER, bool SMOOTH>
 cudaError_t coarse_launch(const CoarsePlan& pl, Dims3 d, float h, const TS* b, const uint32_t* f,
-                          TS* p, int iters, float omega, int bc_mode, cudaStream_t st) {
-  auto kern = k_mg_coarse_rb<TS, K, SYM>;
+                          const uint8_t* meta, TS* p, int iters, float omega, int bc_mode,
+                          cudaStream_t st) {
+  auto kern = k_mg_coarse_rb<TS, K, ORDER, SMOOTH>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        COARSE_SMEM);
   if (e != cudaSuccess) return e;
@@ -440,8 +450,8 @@ cudaError_t coarse_launch(const CoarsePlan& pl, Dims3 d, float h, const TS* b, c
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, kern, Lvl{d.nx, d.ny, d.nz}, h * h, b, f, p, iters, omega,
-                            bc_mode);
+  return cudaLaunchKernelEx(&cfg, kern, Lvl{d.nx, d.ny, d.nz}, h * h, b, f, meta, p, iters,
+                            omega, bc_mode);
 }
 
 // The largest cluster this device co-schedules for the coarse kernel (16
@@ -449,7 +459,7 @@ cudaError_t coarse_launch(const CoarsePlan& pl, Dims3 d, float h, const TS* b, c
 int coarse_max_cluster() {
   static int mc = 0;
   if (mc) return mc;
-  auto kern = k_mg_coarse_rb<float, 2, false>;
+  auto kern = k_mg_coarse_rb<float, 2, RED_BLACK, false>;
   int q = 8;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
           cudaSuccess &&
@@ -472,11 +482,12 @@ cudaError_t mg_coarse_t(Dims3 d, float h, const TS* b, const uint32_t* f, TS* p,
                         float omega, int bc_mode, cudaStream_t st, int symmetric = 0) {
   const CoarsePlan pl = coarse_plan(d, coarse_max_cluster());
   if (pl.C == 0) return cudaErrorInvalidValue;
-#define PYRO_COARSE(K)                                                                          \
-  case K:                                                                                      \
-    return symmetric                                                                           \
-               ? coarse_launch<TS, K, true>(pl, d, h, b, f, p, iters, omega, bc_mode, st)      \
-               : coarse_launch<TS, K, false>(pl, d, h, b, f, p, iters, omega, bc_mode, st)
+#define PYRO_COARSE(K)                                                                       \
+  case K:                                                                                   \
+    return symmetric ? coarse_launch<TS, K, ALTERNATE, false>(pl, d, h, b, f, nullptr, p,   \
+                                                              iters, omega, bc_mode, st)    \
+                     : coarse_launch<TS, K, RED_BLACK, false>(pl, d, h, b, f, nullptr, p,   \
+                                                              iters, omega, bc_mode, st)
   switch (pl.K) {
     PYRO_COARSE(1);
     PYRO_COARSE(2);
@@ -486,9 +497,40 @@ cudaError_t mg_coarse_t(Dims3 d, float h, const TS* b, const uint32_t* f, TS* p,
 #undef PYRO_COARSE
 }
 
+template <typename TS>
+cudaError_t mg_sweeps_t(Dims3 d, float h, const TS* b, const uint8_t* meta, TS* p, int iters,
+                        float omega, int black_first, int bc_mode, cudaStream_t st) {
+  const CoarsePlan pl = coarse_plan(d, coarse_max_cluster());
+  if (pl.C == 0 || pl.K != 1) return cudaErrorInvalidValue;
+  return black_first ? coarse_launch<TS, 1, BLACK_RED, true>(pl, d, h, b, nullptr, meta, p, iters,
+                                                             omega, bc_mode, st)
+                     : coarse_launch<TS, 1, RED_BLACK, true>(pl, d, h, b, nullptr, meta, p, iters,
+                                                             omega, bc_mode, st);
+}
+
 }  // namespace
 
 bool mg_coarse_fits(Dims3 d) { return coarse_cluster_size(d) != 0; }
+
+// Levels with one cell of a colour per thread: a launch sets its cells up once
+// for all passes (16 to 32 k cells: MGPCG on 256^3 13.50 -> 13.30 ms, on 75 x
+// 183 x 75 a 4 cm frame 4.96 -> 4.86 ms), but four cells per thread make a pass
+// longer than a launch (32 x 60 x 32 in the V-cycles on 128 x 240 x 128: 1043
+// us against 968 with a launch per pass).
+bool mg_sweeps_fit(Dims3 d) {
+  const CoarsePlan pl = coarse_plan(d, coarse_max_cluster());
+  return pl.C != 0 && pl.K == 1;
+}
+
+cudaError_t launch_mg_sweeps(Dims3 d, float h, const void* b, const uint8_t* meta, void* p,
+                             int iters, float omega, int black_first, int bc_mode, bool bf16,
+                             cudaStream_t st) {
+  if (bf16)
+    return mg_sweeps_t<__nv_bfloat16>(d, h, (const __nv_bfloat16*)b, meta, (__nv_bfloat16*)p,
+                                      iters, omega, black_first, bc_mode, st);
+  return mg_sweeps_t<float>(d, h, (const float*)b, meta, (float*)p, iters, omega, black_first,
+                            bc_mode, st);
+}
 
 cudaError_t launch_mg_resid(Dims3 d, float h, const float* p, const float* b, const uint32_t* f,
                             int bc_mode, float* stats, cudaStream_t st) {

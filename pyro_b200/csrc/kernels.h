@@ -117,6 +117,13 @@ cudaError_t launch_mg_resid(Dims3 d, float h, const float* p, const float* b, co
                             int bc_mode, float* stats, cudaStream_t st);
 // Whole coarsest-level solve in one CTA (shared memory); returns
 // cudaErrorInvalidValue when the level does not fit.
+// `iters` smoother sweeps (both colours, red first or black first) on a level
+// that fits a thread-block cluster, in one launch; equal to launch_mg_pass /
+// launch_mg_pass_bf16 once per colour, bit for bit.
+bool mg_sweeps_fit(Dims3 d);
+cudaError_t launch_mg_sweeps(Dims3 d, float h, const void* b, const uint8_t* meta, void* p,
+                             int iters, float omega, int black_first, int bc_mode, bool bf16,
+                             cudaStream_t st);
 bool mg_coarse_fits(Dims3 d);
 cudaError_t launch_mg_coarse(Dims3 d, float h, const float* b, const uint32_t* f, float* p,
                              int iters, float omega, int bc_mode, cudaStream_t st);

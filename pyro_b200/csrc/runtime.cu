@@ -54,15 +54,17 @@ cudaError_t MgTimer::start(cudaStream_t st) {
   for (auto e : ev) cudaEventDestroy(e);
   ev.clear();
   cls.clear();
+  steps.clear();
   return mark(-1, st);
 }
 
-cudaError_t MgTimer::mark(int c, cudaStream_t st) {
+cudaError_t MgTimer::mark(int c, cudaStream_t st, int n) {
   cudaEvent_t e;
   cudaError_t r = cudaEventCreate(&e);
   if (r != cudaSuccess) return r;
   ev.push_back(e);
   cls.push_back(c);
+  steps.push_back(n);
   return cudaEventRecord(e, st);
 }
 
@@ -77,7 +79,7 @@ cudaError_t MgTimer::read(float* ms, int* launches) const {
     if (r != cudaSuccess) return r;
     if (cls[i] >= 0 && cls[i] < MG_CLASSES) {
       ms[cls[i]] += t;
-      launches[cls[i]] += 1;
+      launches[cls[i]] += steps[i];
     }
   }
   return cudaSuccess;
@@ -132,6 +134,8 @@ int Multigrid::init(Dims3 d0, float h0, int bc, size_t direct_max) {
     f[l] = own_f[l].as<uint32_t>();
   }
   coarse_one_cta = mg_coarse_fits(dims.back());
+  sweeps_fit.assign(L, 0);
+  for (size_t l = 1; l + 1 < L; l++) sweeps_fit[l] = mg_sweeps_fit(dims[l]) ? 1 : 0;
   return PYRO_OK;
 }
 
@@ -184,12 +188,19 @@ cudaError_t Multigrid::vcycles(int cycles, cudaStream_t st) {
   int nl = (int)dims.size();
   cudaError_t e;
   // with a timer, an event after every launch credits it to its class
-  auto tick = [&](int cls) -> cudaError_t { return timer ? timer->mark(cls, st) : cudaSuccess; };
+  auto tick = [&](int cls, int steps = 1) -> cudaError_t {
+    return timer ? timer->mark(cls, st, steps) : cudaSuccess;
+  };
   if (timer && (e = timer->start(st)) != cudaSuccess) return e;
   if ((e = prepare(st)) != cudaSuccess) return e;
   if ((e = tick(MG_PREPARE)) != cudaSuccess) return e;
   auto M = [&](int l) { return meta[l].as<uint8_t>(); };
   auto sm = [&](int l) -> cudaError_t {  // two red-black iterations, omega 1
+    if (sweeps_fit[l]) {
+      cudaError_t e2 = launch_mg_sweeps(dims[l], h[l], b[l], M(l), phi[l], 2, 1.0f, 0, bc_mode,
+                                        false, st);
+      return e2 == cudaSuccess ? tick(MG_PASS_MID, 4) : e2;
+    }
     for (int it = 0; it < 2; it++)
       for (int c = 0; c < 2; c++) {
         cudaError_t e2 = launch_mg_pass(dims[l], h[l], b[l], M(l), phi[l], c, 1.0f, bc_mode, st);
@@ -251,7 +262,9 @@ cudaError_t Multigrid::vcycle_sym(cudaStream_t st, DevBuf* bphi, DevBuf* bphi2, 
     }
   }
   // with a timer, an event after every step credits it to its class
-  auto tick = [&](int cls) -> cudaError_t { return timer ? timer->mark(cls, st) : cudaSuccess; };
+  auto tick = [&](int cls, int steps = 1) -> cudaError_t {
+    return timer ? timer->mark(cls, st, steps) : cudaSuccess;
+  };
   if (prep && (e = prepare_sym(st)) != cudaSuccess) return e;
   if (prep && (e = tick(MG_PREPARE)) != cudaSuccess) return e;
   auto M = [&](int l) { return meta[l].as<uint8_t>(); };
@@ -278,8 +291,16 @@ cudaError_t Multigrid::vcycle_sym(cudaStream_t st, DevBuf* bphi, DevBuf* bphi2, 
               : launch_mg_pass(dims[l], h[l], (const float*)B(l), M(l), (float*)P(l), c, om,
                                bc_mode, st);
   };
+  // all sweeps of a level that fits a cluster, before or after its correction
+  auto sweeps = [&](int l, int black_first) -> cudaError_t {
+    const int n = sym_sweeps(l);
+    cudaError_t e2 = launch_mg_sweeps(dims[l], h[l], B(l), M(l), P(l), n, kSymOmega, black_first,
+                                      bc_mode, lo, st);
+    return e2 == cudaSuccess ? tick(MG_PASS_MID, 2 * n) : e2;
+  };
   for (int l = 0; l < nl - 1; l++) {
-    for (int it = 0; it < sym_sweeps(l); it++)
+    if (sweeps_fit[l] && (e = sweeps(l, 0)) != cudaSuccess) return e;
+    for (int it = 0; it < sym_sweeps(l) && !sweeps_fit[l]; it++)
       for (int c = 0; c < 2; c++) {
         e = (fuse && l == 0 && it == 0 && c == 0)
                 ? launch_mg_pass_first(dims[0], h[0], b[0], lo ? bb[0].p : nullptr, M(0), P(0), 0,
@@ -317,7 +338,8 @@ cudaError_t Multigrid::vcycle_sym(cudaStream_t st, DevBuf* bphi, DevBuf* bphi2, 
                                  dims[l + 1], M(l + 1), st);
     if (e == cudaSuccess) e = tick(l == 0 ? MG_PROLONG_L0 : MG_PROLONG_MID);
     if (e != cudaSuccess) return e;
-    for (int it = 0; it < sym_sweeps(l); it++)
+    if (sweeps_fit[l] && (e = sweeps(l, 1)) != cudaSuccess) return e;
+    for (int it = 0; it < sym_sweeps(l) && !sweeps_fit[l]; it++)
       for (int c = 1; c >= 0; c--) {
         e = (fuse && lo && l == 0 && it == sym_sweeps(0) - 1 && c == 0)
                 ? launch_mg_pass_last_f32(dims[0], h[0], B(0), M(0), P(0), phi[0], 0, kSymOmega,

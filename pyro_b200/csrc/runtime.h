@@ -67,10 +67,11 @@ enum MgClass {
 // class.  Read after the stream has finished.
 struct MgTimer {
   std::vector<cudaEvent_t> ev;
-  std::vector<int> cls;
+  std::vector<int> cls, steps;
   ~MgTimer();
   cudaError_t start(cudaStream_t st);
-  cudaError_t mark(int c, cudaStream_t st);
+  // steps: the passes that the launch ran
+  cudaError_t mark(int c, cudaStream_t st, int steps = 1);
   // per-class totals (ms) and launch counts
   cudaError_t read(float* ms, int* launches) const;
 };
@@ -102,6 +103,7 @@ struct Multigrid {
   std::vector<DevBuf> meta;   // per-cell neighbour mask (k_mgf.cu)
   std::vector<DevBuf> wq;     // 64 x prolongation weight sums (vcycle_sym, levels < last)
   bool coarse_one_cta = false;
+  std::vector<char> sweeps_fit;  // levels whose sweeps run as one cluster launch
   float* stats = nullptr;  // device, for mg_resid
 
   // direct_max == 0: the reference rule; else the deep rule.

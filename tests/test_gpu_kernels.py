@@ -377,6 +377,36 @@ def test_mg_symmetric_restriction_is_the_adjoint_of_the_prolongation(lib, nx, ny
             assert np.abs(lo - hi).max() <= 2e-2 * np.abs(hi).max()
 
 
+@pytest.mark.parametrize("nx,ny,nz", [(2, 2, 2), (19, 46, 19), (32, 32, 32), (20, 40, 20),
+                                      (7, 9, 3), (64, 31, 16), (64, 31, 17)])
+@pytest.mark.parametrize("bc_mode", [0, 1])
+@pytest.mark.parametrize("storage", [_abi.MG_F32, _abi.MG_BF16])
+def test_mg_sweeps_equal_separate_passes(lib, nx, ny, nz, bc_mode, storage):
+    """The cluster launch of a smoother's sweeps, in both colour orders,
+    against one pass launch per colour: the same bits, the rounding to BF16
+    after every pass included."""
+    rng = np.random.default_rng(nx * ny + nz)
+    enc = _bf16_bits if storage == _abi.MG_BF16 else np.ascontiguousarray
+    f = dev((rng.random((nz, ny, nx)) < 0.15).astype(np.uint32))
+    b = dev(enc(rng.normal(0, 1, (nz, ny, nx)).astype(np.float32)))
+    p = enc(rng.normal(0, 1, (nz, ny, nx)).astype(np.float32))
+    meta = dev(np.zeros((nz, ny, nx), np.uint8))
+    assert lib.pyro_k_mg_meta(nx, ny, nz, ptr(f), ptr(meta), None) == 0
+    for black, sweeps, om in ((0, 2, 1.0), (0, 4, 1.3), (1, 3, 1.3)):
+        want, got = dev(p), dev(p)
+        if (nx + 1) // 2 * ny * -(-nz // 16) > 1024:  # two cells of a colour per thread
+            assert lib.pyro_k_mg_sweeps(nx, ny, nz, 0.2, ptr(b), ptr(meta), ptr(got), sweeps, om,
+                                        black, bc_mode, storage, None) == _abi.PYRO_E_INVALID
+            continue
+        for _ in range(sweeps):
+            for c in ((1, 0) if black else (0, 1)):
+                assert lib.pyro_k_mg_pass(nx, ny, nz, 0.2, ptr(b), ptr(meta), ptr(want), c, om,
+                                          bc_mode, storage, None) == 0
+        assert lib.pyro_k_mg_sweeps(nx, ny, nz, 0.2, ptr(b), ptr(meta), ptr(got), sweeps, om,
+                                    black, bc_mode, storage, None) == 0, lib.pyro_last_error()
+        assert np.array_equal(host(got), host(want)), (black, sweeps)
+
+
 # slabs of one to three planes per CTA of the cluster (nz = 3: three CTAs)
 COARSE_CASES = MG_CASES + [(8, 20, 8, 3, 0.32), (32, 32, 22, 4, 0.2), (20, 40, 20, 5, 0.16),
                            (16, 30, 16, 6, 0.16), (20, 40, 17, 7, 0.16), (12, 20, 3, 11, 0.3)]
