@@ -278,3 +278,34 @@ def test_mgpcg_sealed_pockets(lib, mode):
     assert rel <= 1.5e-6, rel
     assert abs(rel - info.rel_resid) <= 1e-7
     ps.close()
+
+
+@pytest.mark.parametrize("dims", [(24, 30, 18),    # rows of 4-cell chunks
+                                  (26, 30, 18),    # 2-cell chunks, cells a multiple of 4
+                                  (27, 28, 17),    # single cells in rows, 4 in the vectors
+                                  (27, 29, 31)])   # single cells throughout
+@pytest.mark.parametrize("offset", [0, 1])         # floats off a 16-byte boundary
+def test_cg_vector_kernel_forms(lib, dims, offset):
+    """MGPCG against the FP64 solution in every form of the CG vector kernels
+    and for a solution array at any 4-byte alignment: a residual of 1e-6
+    leaves the solution within 1e-3 of its norm (the level-0 condition number
+    of these grids is below 10^3)."""
+    import torch
+
+    from pyro_b200.poisson import PoissonSolver, poisson_case
+    nx, ny, nz = dims
+    f, b = poisson_case(nx, ny, nz, seed=nx, solid=0.05, edge=(1, 3))
+    x, _, _ = oracle.poisson_f64((nx, ny, nz), 0.1, b, f)
+    ps = PoissonSolver((nx, ny, nz), 0.1, 0)
+    ps.set_flags(dev(f).data_ptr())
+    buf = torch.zeros(b.size + 4, dtype=torch.float32, device="cuda")
+    phi = buf[offset:offset + b.size]
+    bd = dev(b)
+    torch.cuda.synchronize()
+    info = ps.solve(bd.data_ptr(), phi.data_ptr(), _abi.SOLVER_MGPCG, 1e-6, 100)
+    assert info.converged and info.rel_resid <= 1e-6
+    got = host(phi).reshape(b.shape).astype(np.float64)
+    fl = f == 0
+    assert np.linalg.norm((got - x)[fl]) <= 1e-3 * np.linalg.norm(x[fl])
+    assert not host(buf[offset + b.size:]).any() and not host(buf[:offset]).any()
+    ps.close()
