@@ -51,6 +51,7 @@
 
 #include <algorithm>
 
+#include "common.cuh"
 #include "conv.cuh"
 #include "net.h"
 #include "umma.cuh"
@@ -71,6 +72,7 @@ struct C3Geom {
   int groups, stages;    // groups of 16 input channels
   int K, CO, N, rb;      // input channels of w, channels per CTA, columns, rows of a weight tap
   int flip;              // packed: 1 when the plane's shifts run backwards
+  int late_w;            // the kernel before may have written the weights
   uint32_t wbytes, ncols;
 };
 
@@ -112,7 +114,11 @@ __global__ void __launch_bounds__(C3_THREADS, 1)
   if (warp == 1) {
     umma::tmem_alloc(&tslot, g.ncols);
     umma::tmem_relinquish();
+    // Only now: a CTA of the next launch on this SM allocates TMEM before it
+    // waits for this launch, so this one must hold its own already.
+    pdl_trigger();
   }
+  if (g.late_w) pdl_wait();
   // ---- weights: [group][K step][chunk][row of rb][8 channels]; row = plane
   // * CO + co, plane p holding tap z = ZO + 1 - p where that is 0, 1 or 2
   for (int c = threadIdx.x; c < C3_MAX_CO; c += C3_THREADS)
@@ -149,6 +155,10 @@ __global__ void __launch_bounds__(C3_THREADS, 1)
   umma::fence_before();
   __syncthreads();
   umma::fence_after();
+  // Up to here nothing that the kernel before may still write: the weights are
+  // laid out while it ends (unless late_w).  The whole network on 32 x 80 x 32
+  // voxels: 172 -> 132 us.
+  pdl_wait();
   const uint32_t tbase = tslot;
   const int my_tiles =
       (int)blockIdx.x < g.ntiles ? (g.ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
@@ -447,7 +457,8 @@ C3Plan c3_plan(int nx, int ny, int nz, int nb, int groups, int N_out, bool pack,
 // N <= 128 output channels.  x must be 16-byte aligned.
 cudaError_t conv3_tma(const bf16* x, int K, int pack, int nx, int ny, int nz, int nb,
                       const bf16* w_tap, int N, const float* bias, int relu, const bf16* mask,
-                      bf16* y_bf16, float* y_f32, int* err, cudaStream_t st, const NetVol* fine) {
+                      bf16* y_bf16, float* y_f32, int* err, cudaStream_t st, const NetVol* fine,
+                      bool old_weights) {
   if (fine && (!y_bf16 || N % 16)) return cudaErrorInvalidValue;
   if ((pack ? K < 1 || K > 2 : K % 16 != 0) || N < 1 || N > C3_MAX_CO)
     return cudaErrorInvalidValue;
@@ -463,6 +474,7 @@ cudaError_t conv3_tma(const bf16* x, int K, int pack, int nx, int ny, int nz, in
   g.nb = nb;
   g.K = K;
   g.flip = pack < 0;
+  g.late_w = old_weights ? 0 : 1;
   g.groups = pack ? 1 : K / 16;
   const C3Plan pl = c3_plan(nx, ny, nz, nb, g.groups, N, pack != 0, nsm);
   if (!pl.zo) return cudaErrorInvalidValue;
@@ -503,8 +515,8 @@ cudaError_t conv3_tma(const bf16* x, int K, int pack, int nx, int ny, int nz, in
              fine ? 1 : 0, fine ? fine->nx : 0, fine ? fine->ny : 0, fine ? fine->nz : 0,
              fine ? (int)fine->voxels() : 0};
   const int ctas = std::max(1, std::min(g.ntiles, nsm / pl.split));
-  kern<<<dim3((unsigned)ctas, (unsigned)pl.split), C3_THREADS, smem, st>>>(tx, w_tap, g, ep, err);
-  return cudaGetLastError();
+  return launch_pdl(kern, dim3((unsigned)ctas, (unsigned)pl.split), dim3(C3_THREADS), smem, st, tx,
+                    w_tap, g, ep, err);
 }
 
 }  // namespace pyro

@@ -13,6 +13,7 @@
 #include <random>
 #include <vector>
 
+#include "common.cuh"
 #include "net.h"
 
 namespace pyro {
@@ -145,6 +146,8 @@ __global__ void __launch_bounds__(NT) k_input(const float* __restrict__ b,
                                               const uint32_t* __restrict__ f, size_t cells,
                                               int nx, int nb, const double* __restrict__ sc,
                                               uint4* __restrict__ in0) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ double inv[MAX_VOLS];
   load_rms(sc, nb, inv);
   if ((int)threadIdx.x < nb) {  // -1: no volume to scale by, its values are 0
@@ -190,6 +193,8 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 // coarse[cv][c] = mean of the children inside the fine volume
 __global__ void __launch_bounds__(NT) k_pool(const bf16* __restrict__ in, int C, Dv fd,
                                              bf16* __restrict__ out) {
+  pdl_trigger();
+  pdl_wait();
   Dv cd{(fd.nx + 1) / 2, (fd.ny + 1) / 2, (fd.nz + 1) / 2, fd.nb};
   const int ch = C / 8;
   GRID_LOOP(i, cd.voxels() * ch) {
@@ -340,6 +345,8 @@ __global__ void __launch_bounds__(NT) k_output(const float* __restrict__ out,
                                                const uint32_t* __restrict__ f, size_t cells,
                                                int nb, const double* __restrict__ sc, double scale,
                                                float* __restrict__ phi) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ double rms[MAX_VOLS];
   load_rms(sc, nb, rms);
   GRID_LOOP(i, cells * nb) {
@@ -576,26 +583,31 @@ int PyroNet::forward(const float* b, const uint32_t* flags, NetVol v, cudaStream
   NET_CU(cudaMemsetAsync(scal.p, 0, scal.bytes, st));
   k_stats<<<dim3(std::min<unsigned>(blocks_for(cells), 148 * 8), v.nb), NT, 0, st>>>(b, flags,
                                                                                     cells, S);
-  k_input<<<std::min(blocks_for(cells * v.nb), 148u * 8u), NT, 0, st>>>(b, flags, cells, v.nx, v.nb, S,
-                                                   in0.as<uint4>());
   NET_CU(cudaGetLastError());
+  // From here each launch may start while the one before it ends
+  // (launch_pdl); k_stats, a plain launch, orders them behind whatever wrote
+  // the weights.
+  NET_CU(launch_pdl(k_input, dim3(std::min(blocks_for(cells * v.nb), 148u * 8u)), dim3(NT), 0, st, b,
+                    flags, cells, v.nx, v.nb, (const double*)S, in0.as<uint4>()));
   // fine != null: the layer's output goes, copied to the children of every
   // voxel, into the first planes of a tensor over the finer volume
   auto conv = [&](const bf16* x, int l, NetVol g, bf16* y, float* yf,
                   const NetVol* fine = nullptr) -> cudaError_t {
     const NetLayer& L = NET_SPEC[l];
     return conv3_tma(x, L.cin, L.cin % 16 ? 1 : 0, g.nx, g.ny, g.nz, g.nb, wf(l), L.cout, bias(l),
-                     L.relu, nullptr, y, yf, E, st, fine);
+                     L.relu, nullptr, y, yf, E, st, fine, true);
   };
   auto B = [](const DevBuf& d) { return d.as<bf16>(); };
   // the skip connections e0, e1 are written straight into their planes of
   // the concatenations c0, c1
   NET_CU(conv(B(in0), 0, v, B(e0a), nullptr));
   NET_CU(conv(B(e0a), 1, v, skip0(), nullptr));
-  k_pool<<<blocks_for(v1.voxels() * 2), NT, 0, st>>>(skip0(), 16, dv(v), B(p1));
+  NET_CU(launch_pdl(k_pool, dim3(blocks_for(v1.voxels() * 2)), dim3(NT), 0, st,
+                    (const bf16*)skip0(), 16, dv(v), B(p1)));
   NET_CU(conv(B(p1), 2, v1, B(e1a), nullptr));
   NET_CU(conv(B(e1a), 3, v1, skip1(), nullptr));
-  k_pool<<<blocks_for(v2.voxels() * 4), NT, 0, st>>>(skip1(), 32, dv(v1), B(p2));
+  NET_CU(launch_pdl(k_pool, dim3(blocks_for(v2.voxels() * 4)), dim3(NT), 0, st,
+                    (const bf16*)skip1(), 32, dv(v1), B(p2)));
   NET_CU(conv(B(p2), 4, v2, B(e2a), nullptr));
   NET_CU(conv(B(e2a), 5, v2, B(c1), nullptr, &v1));
   NET_CU(conv(B(c1), 6, v1, B(c0), nullptr, &v));
@@ -606,9 +618,9 @@ int PyroNet::forward(const float* b, const uint32_t* flags, NetVol v, cudaStream
 
 int PyroNet::output(const uint32_t* flags, float h, float* phi, NetVol v, cudaStream_t st) {
   const size_t cells = (size_t)v.nx * v.ny * v.nz;
-  k_output<<<std::min(blocks_for(cells * v.nb), 148u * 8u), NT, 0, st>>>(out.as<float>(), flags, cells, v.nb,
-                                                    scal.as<double>(),
-                                                    (double)out_scale * h * h, phi);
+  NET_CU(launch_pdl(k_output, dim3(std::min(blocks_for(cells * v.nb), 148u * 8u)), dim3(NT), 0, st,
+                    (const float*)out.as<float>(), flags, cells, v.nb,
+                    (const double*)scal.as<double>(), (double)out_scale * h * h, phi));
   NET_CU(cudaGetLastError());
   return PYRO_OK;
 }
@@ -657,7 +669,7 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
     const bool one = L.cout == 1;
     return conv3_tma(one ? pk.as<bf16>() : dz.as<bf16>(), L.cout, one ? -1 : 0, g.nx, g.ny, g.nz,
                      g.nb, wb(l), L.cin, nullptr, 0, act ? act->as<bf16>() : nullptr,
-                     dx.as<bf16>(), nullptr, E, st);
+                     dx.as<bf16>(), nullptr, E, st, nullptr, true);
   };
   NET_CU(conv3_pack_dx(g9.as<bf16>(), v.nx, v.ny, v.nz, v.nb, -1, pk.as<bf16>(), st));
   NET_CU(wg(d0, g9, 8, v));

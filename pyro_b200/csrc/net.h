@@ -59,12 +59,14 @@ cudaError_t conv3_direct(const __nv_bfloat16* x, int C, int nx, int ny, int nz, 
 // 8 channels, channel j K + k holding voxel u + pack (j - 1).  fine (BF16
 // output of a multiple of 16 channels): every voxel's result is written to its
 // children in the first planes of a tensor over that volume, y_bf16.
+// old_weights: weights and bias were complete before the launch that precedes
+// this one on the stream started, so they may be read while it ends.
 cudaError_t conv3_prep_weights(const __nv_bfloat16* w, int Cout, int Cin, int backward,
                                __nv_bfloat16* w_tap, cudaStream_t st);
 cudaError_t conv3_tma(const __nv_bfloat16* x, int K, int pack, int nx, int ny, int nz, int nb,
                       const __nv_bfloat16* w_tap, int N, const float* bias, int relu,
                       const __nv_bfloat16* mask, __nv_bfloat16* y_bf16, float* y_f32, int* err,
-                      cudaStream_t st, const NetVol* fine = nullptr);
+                      cudaStream_t st, const NetVol* fine = nullptr, bool old_weights = false);
 
 // The driver's cuTensorMapEncodeTiled (PFN_cuTensorMapEncodeTiled_v12000), or
 // null.
