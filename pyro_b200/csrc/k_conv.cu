@@ -465,7 +465,9 @@ cudaError_t conv3_backward_data(const bf16* dy, int Cout, int nx, int ny, int nz
 // by the caller).
 cudaError_t conv3_backward_weight(const bf16* x, int Cin, const bf16* dy, int Cout, int nx,
                                   int ny, int nz, int nb, float* dw, int* err, cudaStream_t st) {
-  if (conv3_wgrad_fits(Cin, Cout))
+  // the boxes need 16-byte aligned tensors; others are gathered
+  const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy);
+  if (conv3_wgrad_fits(Cin, Cout) && at % 16 == 0)
     return conv3_wgrad_tma(x, Cin, dy, Cout, 0, nx, ny, nz, nb, dw, err, st);
   Vol g{nx, ny, nz, nb};
   int V = nx * ny * nz * nb;

@@ -267,7 +267,10 @@ __global__ void __launch_bounds__(C3_THREADS, 1)
     // is (zo, channel).  Two warps share the lanes of a quarter of D and take
     // its pairs of 16-column groups in turn.
     const int q = warp & 3, m = q * 32 + lane, half = (warp - 2) >> 2;
-    const bool planes = ep.out_bf16 && !(ep.Nout & 7) && !(g.CO & 15);
+    // whole 8-channel chunks, 16-byte accesses of the output and the mask
+    const bool planes = ep.out_bf16 && !(ep.Nout & 7) && !(g.CO & 15) &&
+                        !((reinterpret_cast<uintptr_t>(ep.out_bf16) |
+                           reinterpret_cast<uintptr_t>(ep.mask)) & 15);
     const int gpz = g.CO >> 4;  // 16-column groups per output plane
     for (int jt = 0; jt < my_tiles; jt++) {
       const int a = jt & 1;

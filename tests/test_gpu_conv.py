@@ -131,6 +131,28 @@ def test_backward_weight_tma(lib, Cin, Cout, dims, nb):
     _close(dw - 0.5, ref)
 
 
+@pytest.mark.parametrize("off", [(1, 0), (0, 1), (2, 4)])
+def test_backward_weight_unaligned(lib, off):
+    """Tensors that start off a 16-byte boundary are gathered: the same sums."""
+    nb, Cin, Cout, (nz, ny, nx) = 1, 16, 32, (5, 6, 7)
+    x, w, _ = _tensors(nb, Cin, nz, ny, nx, Cout, 14)
+    g = torch.Generator().manual_seed(15)
+    dy = torch.randn(nb, Cout, nz, ny, nx, generator=g).bfloat16().float().cuda()
+    wr = w.clone().requires_grad_(True)
+    Fn.conv3d(x, wr, None, padding=1).backward(dy)
+    ref = wr.grad.permute(0, 2, 3, 4, 1).reshape(Cout, 27, Cin)
+    moved = []
+    for t, o in zip((_cl(x), _cl(dy)), off):
+        m = torch.zeros(t.numel() + 8, dtype=t.dtype, device="cuda")
+        m[o:o + t.numel()] = t.reshape(-1)
+        moved.append(m[o:])
+    dw = torch.zeros((Cout, 27, Cin), dtype=torch.float32, device="cuda")
+    rc = lib.pyro_conv3_backward_weight(ptr(moved[0]), Cin, ptr(moved[1]), Cout, nx, ny, nz, nb,
+                                        ptr(dw), None)
+    assert rc == 0, lib.pyro_last_error()
+    _close(dw, ref)
+
+
 @pytest.mark.parametrize("C,Cout,dims,nb", [
     (16, 16, (1, 1, 1), 1),      # a single voxel
     (16, 16, (5, 17, 9), 2),     # ragged in every direction, two volumes
