@@ -321,3 +321,38 @@ def test_renderer_frame_vs_oracle_chain(lib):
     bad = (np.abs(img - want) > 2e-3 * scale).any(axis=2)
     assert bad.mean() <= 0.05, bad.mean()
     assert abs(img.sum() - want.sum()) <= 3e-2 * np.abs(want).sum()
+
+
+def test_passes_under_stream_capture(lib):
+    """The caches and the camera rays, with the scratch memory their launches
+    take, captured into a CUDA graph: a replay gives the eager calls' bits."""
+    nx, ny, nz = 24, 40, 20
+    P, d = _glowing_frame(nx, ny, nz, seed=11)
+    rp = _abi.PyroRenderParams.from_rows(_rp_rows(P, 32, 20, 2, 7, True))
+    b = _bind(d)
+    lvd, gres = (12, 20, 10), 16
+
+    def frame(stream):
+        render.lightvol(rp, *_args(b), lvd, A, B, rays=4, stream=stream)
+        render.lightground(rp, *_args(b), gres, G, rays=4, stream=stream)
+        render.trace(rp, *_args(b), A, B, lvd, G, gres, acc, stream=stream)
+
+    A, B = _half_empty((10, 20, 12, 4)), _half_empty((10, 20, 12, 4))
+    G = _half_empty((1, gres, gres, 4))
+    acc = torch.zeros((32 * 20, 4), dtype=torch.float32, device="cuda")
+    frame(torch.cuda.current_stream().cuda_stream)
+    want = [host(t).copy() for t in (A, B, G, acc)]
+    for t in (A, B, G):
+        t.fill_(float("nan"))
+    acc.zero_()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        frame(torch.cuda.current_stream().cuda_stream)
+    for _ in range(2):
+        acc.zero_()
+        g.replay()
+    torch.cuda.synchronize()
+    for t, w in zip((A, B, G, acc), want):
+        assert np.array_equal(_bits(host(t)) if t.dtype == torch.float16 else host(t),
+                              _bits(w) if t.dtype == torch.float16 else w)
