@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "common.cuh"
 #include "conv.cuh"
 #include "net.h"
 #include "umma.cuh"
@@ -281,8 +282,12 @@ cudaError_t gemm_dispatch(int npad, dim3 grid, const Load& ld, const Epi& ep, in
 
 
 // --------------------------------------------------------- direct (CUDA cores)
-// 2 -> 16 channels on [voxel][2] inputs (the public entry; the network packs
-// its input for the tensor cores).
+// The two narrow layers, 2 -> 16 channels on [voxel][2] inputs and 16 -> 1,
+// whose sums stay FP32 fused multiply-adds in one fixed order: the tensor
+// cores' sums are faster (160 x 320 x 160 voxels: 2 -> 16 101 us instead of
+// 420, 16 -> 1 159 instead of 491) but further from 64 bits (normal inputs:
+// 16 -> 1 4.1e-7 against 1.5e-7, 2 -> 16 7.0e-8 against 5.2e-8), and the first
+// layer's rounding travels through all that follow.
 // A thread computes DV consecutive voxels of an x-row.  For every (dz, dy)
 // input row it loads the DV + 2 voxels x0-1 .. x0+DV once (zero outside
 // the volume), and the three dx taps of all DV outputs read them from
@@ -300,6 +305,8 @@ __global__ void __launch_bounds__(256, 2) k_conv_direct(const bf16* __restrict__
                                                      const float* __restrict__ bias, int relu,
                                                      bf16* __restrict__ y_bf16,
                                                      float* __restrict__ y_f32) {
+  pdl_trigger();
+  pdl_wait();
   static_assert(CIN == 2 || CIN % 8 == 0, "input rows are loaded as 4- or 16-byte chunks");
   constexpr int DV = DirectShape<CIN, COUT>::DV, CC = DirectShape<CIN, COUT>::CC;
   __shared__ __align__(16) float ws[27 * CIN * COUT];
@@ -486,8 +493,9 @@ cudaError_t conv3_backward_weight(const bf16* x, int Cin, const bf16* dy, int Co
 }
 
 
-// Direct convolution for 2 -> 16 channels; cudaErrorInvalidValue for others.
-bool conv3_direct_fits(int C, int Cout) { return C == 2 && Cout == 16; }
+// Direct convolution for the shapes k_conv_direct covers (2 -> 16 and
+// 16 -> 1 channels); cudaErrorInvalidValue for others.
+bool conv3_direct_fits(int C, int Cout) { return (C == 2 && Cout == 16) || (C == 16 && Cout == 1); }
 
 cudaError_t conv3_direct(const bf16* x, int C, int nx, int ny, int nz, int nb, const bf16* w,
                          int Cout, const float* bias, int relu, bf16* y_bf16, float* y_f32,
@@ -497,11 +505,12 @@ cudaError_t conv3_direct(const bf16* x, int C, int nx, int ny, int nz, int nb, c
     return (unsigned)(((long)((nx + dv - 1) / dv) * ny * nz * nb + 255) / 256);
   };
   if (C == 2 && Cout == 16)
-    k_conv_direct<2, 16><<<blocks(DirectShape<2, 16>::DV), 256, 0, st>>>(x, g, w, bias, relu,
-                                                                         y_bf16, y_f32);
-  else
-    return cudaErrorInvalidValue;
-  return cudaGetLastError();
+    return launch_pdl(k_conv_direct<2, 16>, dim3(blocks(DirectShape<2, 16>::DV)), dim3(256), 0, st,
+                      x, g, w, bias, relu, y_bf16, y_f32);
+  if (C == 16 && Cout == 1)
+    return launch_pdl(k_conv_direct<16, 1>, dim3(blocks(DirectShape<16, 1>::DV)), dim3(256), 0, st,
+                      x, g, w, bias, relu, y_bf16, y_f32);
+  return cudaErrorInvalidValue;
 }
 
 // Weight layouts for conv3_tma: forward w_tap[t][co][ci] = w[co][t][ci];
@@ -564,7 +573,7 @@ int pyro_conv3_forward(const void* x, int C, int nx, int ny, int nz, int nb, con
     if ((rc = wt.alloc((size_t)Cout * 27 * C * 2)) != PYRO_OK) return rc;
     e = conv3_prep_weights((const bf16*)w, Cout, C, 0, wt.as<bf16>(), st);
     if (e == cudaSuccess)
-      e = conv3_tma((const bf16*)x, C, 0, nx, ny, nz, nb, wt.as<bf16>(), Cout, bias, relu, nullptr,
+      e = conv3_tma((const bf16*)x, C, false, nx, ny, nz, nb, wt.as<bf16>(), Cout, bias, relu, nullptr,
                     y_f32 ? nullptr : (bf16*)y, y_f32 ? (float*)y : nullptr, err.as<int>(), st);
     return finish(e, err, st, "pyro_conv3_forward");
   }
@@ -590,7 +599,7 @@ int pyro_conv3_backward_data(const void* dy, int Cout, int nx, int ny, int nz, i
     if ((rc = wt.alloc((size_t)Cout * 27 * Cin * 2)) != PYRO_OK) return rc;
     e = conv3_prep_weights((const bf16*)w, Cout, Cin, 1, wt.as<bf16>(), st);
     if (e == cudaSuccess)
-      e = conv3_tma((const bf16*)dy, Cout, 0, nx, ny, nz, nb, wt.as<bf16>(), Cin, nullptr, 0,
+      e = conv3_tma((const bf16*)dy, Cout, false, nx, ny, nz, nb, wt.as<bf16>(), Cin, nullptr, 0,
                     (const bf16*)act, dx_f32 ? nullptr : (bf16*)dx, dx_f32 ? (float*)dx : nullptr,
                     err.as<int>(), st);
     return finish(e, err, st, "pyro_conv3_backward_data");

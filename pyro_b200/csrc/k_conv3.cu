@@ -24,8 +24,8 @@
 //    the rows [zero planes][tap 2][tap 1][tap 0][zero planes] of co channels:
 //    the N rows for input plane zi are the window that starts at plane
 //    ZO + 1 - zi.  The block writes it once from the tap-major weights.
-//  * packed inputs (one plane of 8 channels that holds the three x-shifts of
-//    a 1- or 2-channel tensor): the taps along x are channels,
+//  * a packed input (one plane of 8 channels that holds the three x-shifts of
+//    a 1-channel tensor): the taps along x are channels,
 //    the box has no x halo, and a K step of 16 is two rows y (the tap pairs
 //    (0, 1) and (-, 2), the missing one with zero weights).
 //
@@ -38,10 +38,9 @@
 //
 // Measured on 160 x 320 x 160 voxels against the form this replaces (output
 // channels as the MMA's 128 rows, of which 16 to 64 were used, and three
-// shifted copies of x; 2 -> 16 and 16 -> 1 channels on the CUDA cores), in us:
-// 2 -> 16 405 -> 101, 16 -> 16 773 -> 244, 48 -> 16 1990 -> 598, 16 -> 1 493
-// -> 159; on 80 x 160 x 80, 96 -> 32 522 -> 320; the data gradient 16 -> 48 on
-// two 128^3 volumes 1411 -> 370.  What bounds it now: the MMAs' issue
+// shifted copies of x), in us: 16 -> 16 773 -> 244, 48 -> 16 1990 -> 598; on
+// 80 x 160 x 80, 96 -> 32 522 -> 320; the data gradient 16 -> 48 on two 128^3
+// volumes 1411 -> 370.  What bounds it now: the MMAs' issue
 // (48 -> 16: 54 MMAs of 48 cycles per 512 voxels and group are 0.44 ms at
 // 1.9 GHz; copying the input with cp.async from four warps measured 684 us
 // against 598 with the boxes).
@@ -71,7 +70,6 @@ struct C3Geom {
   int nx, ny, nz, nb, tiles_x, tiles_y, tiles_z, ntiles;
   int groups, stages;    // groups of 16 input channels
   int K, CO, N, rb;      // input channels of w, channels per CTA, columns, rows of a weight tap
-  int flip;              // packed: 1 when the plane's shifts run backwards
   int late_w;            // the kernel before may have written the weights
   uint32_t wbytes, ncols;
 };
@@ -138,11 +136,8 @@ __global__ void __launch_bounds__(C3_THREADS, 1)
         const int dy = t + j;
         if (t == 0 || j == 1) {
           bf16* e = reinterpret_cast<bf16*>(&v);
-          for (int s = 0; s < 3; s++)
-            for (int k = 0; k < g.K; k++)
-              e[s * g.K + k] =
-                  w_tap[((size_t)(tz * 9 + dy * 3 + (g.flip ? 2 - s : s)) * ep.Nout + co) * g.K +
-                        k];
+          for (int s = 0; s < 3; s++)  // channel s holds voxel u - (s - 1)
+            e[s] = w_tap[(size_t)(tz * 9 + dy * 3 + 2 - s) * ep.Nout + co];
         }
       } else {
         v = *reinterpret_cast<const uint4*>(
@@ -455,15 +450,14 @@ C3Plan c3_plan(int nx, int ny, int nz, int nb, int groups, int N_out, bool pack,
 
 // y[v][n] = sum_{t, k} w_tap[t][n][k] x[v + tap(t)][k] (+ bias, ReLU, or
 // zeroed where mask[v][n] <= 0); K (channels of x) a multiple of 16, or with
-// pack = +-1 the K = 1 or 2 channels of a tensor whose x-shifts are packed
-// into one plane of 8 channels, channel j K + k holding voxel u + pack (j - 1);
-// N <= 128 output channels.  x must be 16-byte aligned.
-cudaError_t conv3_tma(const bf16* x, int K, int pack, int nx, int ny, int nz, int nb,
+// pack K = 1 and the x-shifts of a one-channel tensor in one plane of 8
+// channels (conv3_pack_grad); N <= 128 output channels.  x must be 16-byte aligned.
+cudaError_t conv3_tma(const bf16* x, int K, bool pack, int nx, int ny, int nz, int nb,
                       const bf16* w_tap, int N, const float* bias, int relu, const bf16* mask,
                       bf16* y_bf16, float* y_f32, int* err, cudaStream_t st, const NetVol* fine,
                       bool old_weights) {
   if (fine && (!y_bf16 || N % 16)) return cudaErrorInvalidValue;
-  if ((pack ? K < 1 || K > 2 : K % 16 != 0) || N < 1 || N > C3_MAX_CO)
+  if ((pack ? K != 1 : K % 16 != 0) || N < 1 || N > C3_MAX_CO)
     return cudaErrorInvalidValue;
   PFN_cuTensorMapEncodeTiled_v12000 enc = (PFN_cuTensorMapEncodeTiled_v12000)tensor_map_encoder();
   if (!enc) return cudaErrorNotSupported;
@@ -476,10 +470,9 @@ cudaError_t conv3_tma(const bf16* x, int K, int pack, int nx, int ny, int nz, in
   g.nz = nz;
   g.nb = nb;
   g.K = K;
-  g.flip = pack < 0;
   g.late_w = old_weights ? 0 : 1;
   g.groups = pack ? 1 : K / 16;
-  const C3Plan pl = c3_plan(nx, ny, nz, nb, g.groups, N, pack != 0, nsm);
+  const C3Plan pl = c3_plan(nx, ny, nz, nb, g.groups, N, pack, nsm);
   if (!pl.zo) return cudaErrorInvalidValue;
   const int taps = pack ? 2 : 9, px = pack ? TX : TX + 2;
   g.CO = pl.co;
@@ -510,7 +503,7 @@ cudaError_t conv3_tma(const bf16* x, int K, int pack, int nx, int ny, int nz, in
                                         {k_conv3<4, false>, k_conv3<4, true>},
                                         {k_conv3<8, false>, k_conv3<8, true>}};
   const Kern3 kern = kerns[pl.zo == 1 ? 0 : pl.zo == 2 ? 1 : pl.zo == 4 ? 2 : 3][pack ? 1 : 0];
-  const size_t smem = (size_t)g.wbytes + (size_t)g.stages * c3_stage(pl.zo, pack != 0) + 128;
+  const size_t smem = (size_t)g.wbytes + (size_t)g.stages * c3_stage(pl.zo, pack) + 128;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem);
   if (e != cudaSuccess) return e;

@@ -257,16 +257,17 @@ bool encode_planes(CUtensorMap* m, const bf16* p, int planes, int nx, int ny, in
          CUDA_SUCCESS;
 }
 
-// dst[u][j] = src[u + sign (j - 1)] for the three x-shifts j, 0 outside the
-// row and in the channels past 3: a tensor of one channel as a plane of 8.
-__global__ void __launch_bounds__(256) k_pack_dx(const uint16_t* __restrict__ src, size_t V,
-                                                 int nx, int sign, uint4* __restrict__ dst) {
+// conv3_pack_grad and conv3_pack_input: T is a voxel, one or two channels.
+template <typename T>
+__global__ void __launch_bounds__(256) k_pack_dx(const T* __restrict__ src, size_t V, int nx,
+                                                 uint4* __restrict__ dst) {
   const size_t u = blockIdx.x * (size_t)256 + threadIdx.x;
   if (u >= V) return;
   const int x = (int)((uint32_t)u % (uint32_t)nx);
-  const uint32_t lo = (unsigned)(x - sign) < (unsigned)nx ? src[u - sign] : 0u;
-  const uint32_t hi = (unsigned)(x + sign) < (unsigned)nx ? src[u + sign] : 0u;
-  dst[u] = make_uint4(lo | (uint32_t)src[u] << 16, hi, 0u, 0u);
+  const uint32_t left = x > 0 ? src[u - 1] : 0u, mid = src[u],
+                 right = x + 1 < nx ? src[u + 1] : 0u;
+  dst[u] = sizeof(T) == 2 ? make_uint4(right | mid << 16, left, 0u, 0u)
+                          : make_uint4(left, mid, right, 0u);
 }
 
 }  // namespace
@@ -275,11 +276,16 @@ __global__ void __launch_bounds__(256) k_pack_dx(const uint16_t* __restrict__ sr
 // planes of output channels (N a multiple of 16).
 bool conv3_wgrad_fits(int Cin, int Cout) { return Cin % 8 == 0 && Cout % 16 == 0; }
 
-cudaError_t conv3_pack_dx(const bf16* src, int nx, int ny, int nz, int nb, int sign, bf16* dst,
-                          cudaStream_t st) {
+cudaError_t conv3_pack_grad(const bf16* src, int nx, int ny, int nz, int nb, bf16* dst,
+                            cudaStream_t st) {
   const size_t V = (size_t)nx * ny * nz * nb;
-  k_pack_dx<<<(unsigned)((V + 255) / 256), 256, 0, st>>>((const uint16_t*)src, V, nx, sign,
-                                                         (uint4*)dst);
+  k_pack_dx<<<(unsigned)((V + 255) / 256), 256, 0, st>>>((const uint16_t*)src, V, nx, (uint4*)dst);
+  return cudaGetLastError();
+}
+cudaError_t conv3_pack_input(const bf16* src, int nx, int ny, int nz, int nb, bf16* dst,
+                             cudaStream_t st) {
+  const size_t V = (size_t)nx * ny * nz * nb;
+  k_pack_dx<<<(unsigned)((V + 255) / 256), 256, 0, st>>>((const uint32_t*)src, V, nx, (uint4*)dst);
   return cudaGetLastError();
 }
 

@@ -137,38 +137,21 @@ __device__ __forceinline__ void load_rms(const double* sc, int nb, double (&rms)
   __syncthreads();
 }
 
-// The network's input (b / s, solid) as one plane of 8 channels holding its
-// three x-shifts: channels 2 j + {0, 1} of voxel u are the values of voxel
-// u + j - 1, 0 outside the row, so that the first layer and its weight
-// gradient run on the tensor cores (160 x 320 x 160: 72 us with s and three
-// divisions per voxel, 45 us with 1 / s per block).
+// The network's input (b / s, solid) per voxel; 0 where there is no s to scale
+// by (160 x 320 x 160: 31 us).
 __global__ void __launch_bounds__(NT) k_input(const float* __restrict__ b,
                                               const uint32_t* __restrict__ f, size_t cells,
-                                              int nx, int nb, const double* __restrict__ sc,
-                                              uint4* __restrict__ in0) {
+                                              int nb, const double* __restrict__ sc,
+                                              __nv_bfloat162* __restrict__ in0) {
   pdl_trigger();
   pdl_wait();
-  __shared__ double inv[MAX_VOLS];
-  load_rms(sc, nb, inv);
-  if ((int)threadIdx.x < nb) {  // -1: no volume to scale by, its values are 0
-    const double s = inv[threadIdx.x];
-    inv[threadIdx.x] = s > 0.0 ? 1.0 / s : -1.0;
-  }
-  __syncthreads();
+  __shared__ double rms[MAX_VOLS];
+  load_rms(sc, nb, rms);
   GRID_LOOP(i, cells * nb) {
-    const int x = (int)((uint32_t)i % (uint32_t)nx);
-    const double s = inv[(uint32_t)i / (uint32_t)cells];
-    uint32_t w[3];
-#pragma unroll
-    for (int j = 0; j < 3; j++) {
-      const bool in = (unsigned)(x + j - 1) < (unsigned)nx;
-      const size_t k = in ? i + j - 1 : i;
-      const bool solid = __ldg(f + k) == 1u;
-      const float v = solid || s < 0.0 ? 0.0f : (float)((double)__ldg(b + k) * s);
-      const __nv_bfloat162 h = __floats2bfloat162_rn(v, solid ? 1.0f : 0.0f);
-      w[j] = in ? *reinterpret_cast<const uint32_t*>(&h) : 0u;
-    }
-    in0[i] = make_uint4(w[0], w[1], w[2], 0u);
+    const double s = rms[(uint32_t)i / (uint32_t)cells];
+    const bool solid = f[i] == 1u;
+    const float v = !solid && s > 0.0 ? (float)((double)b[i] / s) : 0.0f;
+    in0[i] = __floats2bfloat162_rn(v, solid ? 1.0f : 0.0f);
   }
 }
 
@@ -540,7 +523,7 @@ int PyroNet::ensure(NetVol v, bool bwd) {
     DevBuf* b;
     size_t n;
   };
-  std::vector<A> fw = {{&in0, V0 * 8},  {&e0a, V0 * 16}, {&p1, V1 * 16},
+  std::vector<A> fw = {{&in0, V0 * 2},  {&e0a, V0 * 16}, {&p1, V1 * 16},
                        {&e1a, V1 * 32}, {&p2, V2 * 32}, {&e2a, V2 * 64},
                        {&c1, V1 * 96},  {&c0, V0 * 48}, {&d0, V0 * 16}};
   std::vector<A> bw = {{&g9, V0 * 1},   {&g8, V0 * 16}, {&gc0, V0 * 48}, {&g7, V1 * 32},
@@ -588,14 +571,17 @@ int PyroNet::forward(const float* b, const uint32_t* flags, NetVol v, cudaStream
   // (launch_pdl); k_stats, a plain launch, orders them behind whatever wrote
   // the weights.
   NET_CU(launch_pdl(k_input, dim3(std::min(blocks_for(cells * v.nb), 148u * 8u)), dim3(NT), 0, st, b,
-                    flags, cells, v.nx, v.nb, (const double*)S, in0.as<uint4>()));
+                    flags, cells, v.nb, (const double*)S, in0.as<__nv_bfloat162>()));
   // fine != null: the layer's output goes, copied to the children of every
   // voxel, into the first planes of a tensor over the finer volume
   auto conv = [&](const bf16* x, int l, NetVol g, bf16* y, float* yf,
                   const NetVol* fine = nullptr) -> cudaError_t {
     const NetLayer& L = NET_SPEC[l];
-    return conv3_tma(x, L.cin, L.cin % 16 ? 1 : 0, g.nx, g.ny, g.nz, g.nb, wf(l), L.cout, bias(l),
-                     L.relu, nullptr, y, yf, E, st, fine, true);
+    if (conv3_direct_fits(L.cin, L.cout))
+      return conv3_direct(x, L.cin, g.nx, g.ny, g.nz, g.nb, w(l), L.cout, bias(l), L.relu, y, yf,
+                          st);
+    return conv3_tma(x, L.cin, false, g.nx, g.ny, g.nz, g.nb, wf(l), L.cout, bias(l), L.relu,
+                     nullptr, y, yf, E, st, fine, true);
   };
   auto B = [](const DevBuf& d) { return d.as<bf16>(); };
   // the skip connections e0, e1 are written straight into their planes of
@@ -649,8 +635,9 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
     if (L.cout == 1)  // the last layer: pk holds its gradient's shifts
       e = conv3_wgrad_tma(xs, L.cin, pk.as<bf16>(), 1, 1, g.nx, g.ny, g.nz, g.nb, G + w_off[l], E,
                           st);
-    else if (L.cin == 2)  // the first: in0 holds the input's
-      e = conv3_wgrad_tma(xs, 2, gs, L.cout, 2, g.nx, g.ny, g.nz, g.nb, G + w_off[l], E, st);
+    else if (L.cin == 2)  // the first: pk holds the input's
+      e = conv3_wgrad_tma(pk.as<bf16>(), 2, gs, L.cout, 2, g.nx, g.ny, g.nz, g.nb, G + w_off[l], E,
+                          st);
     else
       e = conv3_backward_weight(xs, L.cin, gs, L.cout, g.nx, g.ny, g.nz, g.nb, G + w_off[l], E,
                                 st);
@@ -667,11 +654,10 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
   auto bd = [&](const DevBuf& dz, int l, NetVol g, const DevBuf* act, DevBuf& dx) -> cudaError_t {
     const NetLayer& L = NET_SPEC[l];
     const bool one = L.cout == 1;
-    return conv3_tma(one ? pk.as<bf16>() : dz.as<bf16>(), L.cout, one ? -1 : 0, g.nx, g.ny, g.nz,
-                     g.nb, wb(l), L.cin, nullptr, 0, act ? act->as<bf16>() : nullptr,
+    return conv3_tma(one ? pk.as<bf16>() : dz.as<bf16>(), L.cout, one, g.nx, g.ny, g.nz, g.nb, wb(l), L.cin, nullptr, 0, act ? act->as<bf16>() : nullptr,
                      dx.as<bf16>(), nullptr, E, st, nullptr, true);
   };
-  NET_CU(conv3_pack_dx(g9.as<bf16>(), v.nx, v.ny, v.nz, v.nb, -1, pk.as<bf16>(), st));
+  NET_CU(conv3_pack_grad(g9.as<bf16>(), v.nx, v.ny, v.nz, v.nb, pk.as<bf16>(), st));
   NET_CU(wg(d0, g9, 8, v));
   NET_CU(bd(g9, 8, v, &d0, g8));
   NET_CU(wg(c0, g8, 7, v));
@@ -697,6 +683,7 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
                                                         32, skip0(), dv(v), g2.as<bf16>());
   NET_CU(wg(e0a, g2, 1, v));
   NET_CU(bd(g2, 1, v, &e0a, g1));
+  NET_CU(conv3_pack_input(in0.as<bf16>(), v.nx, v.ny, v.nz, v.nb, pk.as<bf16>(), st));
   NET_CU(wg(in0, g1, 0, v));
   NET_CU(cudaGetLastError());
   return PYRO_OK;

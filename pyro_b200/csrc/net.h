@@ -18,7 +18,7 @@
 // halves with ceil (a coarse cell averages its children inside the volume);
 // up2 copies a coarse cell to its children.  Activations of C channels are
 // stored as C / 8 planes of [volume][z][y][x][8 channels] (C a multiple of
-// 8); the 2-channel input as one such plane holding its three x-shifts.
+// 8), the 2-channel input as [volume][z][y][x][2].
 #pragma once
 
 #include <cuda_bf16.h>
@@ -47,23 +47,23 @@ cudaError_t conv3_backward_weight(const __nv_bfloat16* x, int Cin, const __nv_bf
                                   int Cout, int nx, int ny, int nz, int nb, float* dw, int* err,
                                   cudaStream_t st);
 
-// Direct convolution on the CUDA cores for 2 -> 16 channels on [V][2] inputs.
+// Direct convolution on the CUDA cores for 2 -> 16 channels on [V][2] inputs
+// and 16 -> 1, FP32 sums in a fixed order.
 bool conv3_direct_fits(int C, int Cout);
 cudaError_t conv3_direct(const __nv_bfloat16* x, int C, int nx, int ny, int nz, int nb,
                          const __nv_bfloat16* w, int Cout, const float* bias, int relu,
                          __nv_bfloat16* y_bf16, float* y_f32, cudaStream_t st);
 
 // TMA-staged convolution (k_conv3.cu) on tap-major weights prepared by
-// conv3_prep_weights: input channels K a multiple of 16, or (pack = +-1) the
-// K = 1 or 2 channels of a tensor whose x-shifts are packed into one plane of
-// 8 channels, channel j K + k holding voxel u + pack (j - 1).  fine (BF16
+// conv3_prep_weights: input channels K a multiple of 16, or (pack) the one
+// channel of a tensor packed by conv3_pack_grad.  fine (BF16
 // output of a multiple of 16 channels): every voxel's result is written to its
 // children in the first planes of a tensor over that volume, y_bf16.
 // old_weights: weights and bias were complete before the launch that precedes
 // this one on the stream started, so they may be read while it ends.
 cudaError_t conv3_prep_weights(const __nv_bfloat16* w, int Cout, int Cin, int backward,
                                __nv_bfloat16* w_tap, cudaStream_t st);
-cudaError_t conv3_tma(const __nv_bfloat16* x, int K, int pack, int nx, int ny, int nz, int nb,
+cudaError_t conv3_tma(const __nv_bfloat16* x, int K, bool pack, int nx, int ny, int nz, int nb,
                       const __nv_bfloat16* w_tap, int N, const float* bias, int relu,
                       const __nv_bfloat16* mask, __nv_bfloat16* y_bf16, float* y_f32, int* err,
                       cudaStream_t st, const NetVol* fine = nullptr, bool old_weights = false);
@@ -74,16 +74,19 @@ void* tensor_map_encoder();
 
 // Weight gradient with TMA-staged operands (k_wgrad.cu), accumulated into dw
 // (FP32): input channels in planes of 8 and output channels a multiple of 16;
-// pack 1: one output channel whose gradient gr is packed by conv3_pack_dx
-// with sign -1; pack 2: two input channels, x packed as the network's input.
+// pack 1: one output channel, gr packed by conv3_pack_grad; pack 2: two input
+// channels, x packed by conv3_pack_input.
 bool conv3_wgrad_fits(int Cin, int Cout);
 cudaError_t conv3_wgrad_tma(const __nv_bfloat16* x, int Cin, const __nv_bfloat16* gr, int Cout,
                             int pack, int nx, int ny, int nz, int nb, float* dw, int* err,
                             cudaStream_t st);
-// The three x-shifts of a tensor of one channel as one plane of 8 channels:
-// dst[u][j] = src[u + sign (j - 1)], 0 outside the row.
-cudaError_t conv3_pack_dx(const __nv_bfloat16* src, int nx, int ny, int nz, int nb, int sign,
-                          __nv_bfloat16* dst, cudaStream_t st);
+// The three x-shifts of a gradient of one channel ([V]) or of an input of two
+// ([V][2]) as one plane of 8 channels, 0 outside the row and past the shifts:
+// dst[u][j] = src[u - (j - 1)], dst[u][2 j + c] = src[u + j - 1][c].
+cudaError_t conv3_pack_grad(const __nv_bfloat16* src, int nx, int ny, int nz, int nb,
+                            __nv_bfloat16* dst, cudaStream_t st);
+cudaError_t conv3_pack_input(const __nv_bfloat16* src, int nx, int ny, int nz, int nb,
+                             __nv_bfloat16* dst, cudaStream_t st);
 
 constexpr int NET_LAYERS = 9;
 struct NetLayer {
@@ -120,7 +123,7 @@ struct PyroNet {
   __nv_bfloat16* skip1() const {
     return c1.as<__nv_bfloat16>() + (size_t)8 * vol.half().voxels() * 8;
   }
-  pyro::DevBuf pk;  // packed x-shifts of the output gradient (backward)
+  pyro::DevBuf pk;  // packed x-shifts of the output gradient, then of the input (backward)
   pyro::DevBuf g9, g8, gc0, g7, gc1, g6, g5, gp2, g4, g3, gp1, g2, g1;
   cudaStream_t stream = nullptr;
 

@@ -185,3 +185,32 @@ def test_forward_tiles(lib, C, Cout, dims, nb):
     else:
         bf = y16.view(nb, nz, ny, nx, Cout).permute(0, 4, 1, 2, 3)
     assert torch.equal(bf, got.bfloat16())
+
+
+@pytest.mark.parametrize("C,Cout,dims", [(2, 16, (5, 7, 11)), (16, 1, (5, 7, 11)),
+                                         (16, 1, (1, 3, 2))])
+def test_narrow_layers_sum_in_fp32_order(lib, C, Cout, dims):
+    """2 -> 16 and 16 -> 1 channels: one FP32 fused multiply-add per product in
+    the order (dz, dy, 8 channels, dx, channel), bit for bit.  Operands kept
+    away from 0 leave every product plus partial sum exact in FP64, so the
+    rounding to FP32 is the fused one."""
+    nz, ny, nx = dims
+    x, w, b = _tensors(1, C, nz, ny, nx, Cout, 21)
+    x = torch.where(x.abs() < 2.0 ** -8, torch.zeros_like(x), x)
+    w = torch.where(w.abs() < 2.0 ** -10, torch.zeros_like(w), w)
+    xp = Fn.pad(x, (1,) * 6).double()
+    acc = b.view(1, -1, 1, 1, 1).expand(1, Cout, nz, ny, nx).clone()
+    for dz in range(3):
+        for dy in range(3):
+            for c0 in range(0, C, 8):
+                for dx in range(3):
+                    for c in range(c0, min(c0 + 8, C)):
+                        s = xp[:, c:c + 1, dz:dz + nz, dy:dy + ny, dx:dx + nx]
+                        p = s * w[:, c, dz, dy, dx].double().view(1, -1, 1, 1, 1)
+                        acc = (p + acc.double()).float()
+    y = torch.empty(1, nz, ny, nx, Cout, dtype=torch.float32, device="cuda")
+    xc, wk = _cl(x), _wk(w)
+    rc = lib.pyro_conv3_forward(ptr(xc), C, nx, ny, nz, 1, ptr(wk), Cout, ptr(b), 0, ptr(y), 1,
+                                None)
+    assert rc == 0, lib.pyro_last_error()
+    assert torch.equal(y.permute(0, 4, 1, 2, 3), acc)

@@ -7,11 +7,12 @@ import numpy as np
 import pytest
 import torch
 
-from gpu_util import dev, host, require_cuda
+from gpu_util import dev, host, ptr, require_cuda
 from oracle import learned as L
 from pyro_b200 import _abi
 from pyro_b200.learned import Net
 from pyro_b200.poisson import PoissonSolver, poisson_case
+from test_gpu_conv import _cl
 
 pytestmark = pytest.mark.gpu
 
@@ -69,6 +70,71 @@ def test_forward_matches_oracle(lib, dims, nb):
     assert _rel(got, ref) < 5e-3
     # the float64 network without BF16 rounding is close too
     assert _rel(got, L.predict(p, b, flags, h)) < 5e-2
+
+
+def _layer(lib, x, w, b, relu, f32):
+    """One layer through its public entry: x (nb, C, z, y, x) FP32 of BF16 values."""
+    nb, C, nz, ny, nx = x.shape
+    co = w.shape[0]
+    xc = _cl(x)
+    wc, bc = w.bfloat16().contiguous(), b.float().contiguous()
+    y = torch.empty(nb * nz * ny * nx * co, dtype=torch.float32 if f32 else torch.bfloat16,
+                    device="cuda")
+    rc = lib.pyro_conv3_forward(ptr(xc), C, nx, ny, nz, nb, ptr(wc), co, ptr(bc), relu, ptr(y),
+                                int(f32), None)
+    assert rc == 0, lib.pyro_last_error()
+    if f32:
+        return y.view(nb, nz, ny, nx, co).permute(0, 4, 1, 2, 3)
+    return (y.view(co // 8, nb, nz, ny, nx, 8).permute(1, 0, 5, 2, 3, 4)
+            .reshape(nb, co, nz, ny, nx).float())
+
+
+@pytest.mark.parametrize("dims,nb", [((6, 9, 13), 2), ((24, 40, 30), 1)])
+def test_forward_is_its_layers_bit_for_bit(lib, dims, nb):
+    """The network against its layers called one by one through the public
+    convolution (whose sums the convolution tests pin), with its pooling,
+    up-sampling, input and output scaling restated: the same bits."""
+    b, flags, _ = _case(8, nb, dims)
+    net, p = _net(9)
+    ws, bs = L.unpack(p)
+    W = [torch.from_numpy(np.ascontiguousarray(w)).float().cuda() for w in ws]
+    B = [torch.from_numpy(np.ascontiguousarray(v)).float().cuda() for v in bs]
+    bd, fd, _ = _dev_case(b, flags, b)
+    fluid = (fd != 1).double()
+    s = ((bd.double() ** 2 * fluid).sum((1, 2, 3)) / fluid.sum((1, 2, 3))).sqrt().view(-1, 1, 1, 1)
+    v = torch.where(fd != 1, (bd.double() / s).float(), torch.zeros_like(bd))
+    x = torch.stack([v, 1.0 - fluid.float()], 1).bfloat16().float()
+
+    def conv(t, l):
+        return _layer(lib, t, W[l], B[l], L.SPEC[l][3], l == 8)
+
+    def pool(t):
+        pad = (0, t.shape[4] & 1, 0, t.shape[3] & 1, 0, t.shape[2] & 1)
+        n = torch.nn.functional.pad(torch.ones_like(t[:1, :1]), pad)
+        t = torch.nn.functional.pad(t, pad)
+        acc, cnt = 0.0, 0.0
+        for k in range(8):  # FP32 sums in the children's order
+            sl = (slice(None), slice(None), slice(k >> 2, None, 2), slice(k >> 1 & 1, None, 2),
+                  slice(k & 1, None, 2))
+            acc, cnt = acc + t[sl], cnt + n[sl]
+        return (acc * (1.0 / cnt)).bfloat16().float()
+
+    def up_cat(t, skip):
+        for d in (2, 3, 4):
+            t = t.repeat_interleave(2, dim=d)
+        return torch.cat([t[:, :, :skip.shape[2], :skip.shape[3], :skip.shape[4]], skip], 1)
+
+    e0 = conv(conv(x, 0), 1)
+    e1 = conv(conv(pool(e0), 2), 3)
+    e2 = conv(conv(pool(e1), 4), 5)
+    out = conv(conv(up_cat(conv(up_cat(e2, e1), 6), e0), 7), 8)[:, 0]
+    h = 0.05
+    scale = net.get_params()[1] * float(np.float32(h)) * float(np.float32(h))
+    want = torch.where(fd != 1, (out.double() * scale * s).float(), torch.zeros_like(bd))
+    phi = torch.empty_like(bd)
+    nz, ny, nx = dims
+    net.forward(bd.data_ptr(), fd.data_ptr(), (nx, ny, nz), nb, h, phi.data_ptr())
+    assert np.array_equal(host(phi), host(want))
 
 
 @pytest.mark.parametrize("w_phi,w_res,scale", [(1.0, 0.0, 1.0), (0.3, 2.0, 2.0)])
