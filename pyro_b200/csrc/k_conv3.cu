@@ -15,6 +15,14 @@
 // 64, 64 for 128), so 16 channels need 27 x 45 cycles per 128 voxels plane by
 // plane and 54 x 48 per 512 with ZO = 4.
 //
+// A zero weight times an input that is not finite is NaN, which such an input
+// would spread over all of the tile's planes.  So a tile whose sums are not
+// all finite is done again at the end, plane by plane with the 27 taps alone
+// (N = co): the sums of the same products in the same order, and so the bits
+// of a volume without it outside the 27 neighbours of such a voxel.  (Windows
+// of three planes' columns would need no zeros, but MMAs on overlapping
+// columns are ordered only where accumulator and shape are the same.)
+//
 //  * x: a stage holds 16 input channels: [2 chunks of 8 channels][ZO + 2
 //    planes][18 rows][10 voxels], a box per chunk and plane, zero-filled
 //    outside the volume.  Rows of A are (y, x): core matrices of 8 voxels,
@@ -23,7 +31,8 @@
 //  * w: resident in shared memory for the whole kernel, per tap (dy, dx) as
 //    the rows [zero planes][tap 2][tap 1][tap 0][zero planes] of co channels:
 //    the N rows for input plane zi are the window that starts at plane
-//    ZO + 1 - zi.  The block writes it once from the tap-major weights.
+//    ZO + 1 - zi.  co is padded to 16 with zero rows.  The block writes it once
+//    from the tap-major weights.
 //  * a packed input (one plane of 8 channels that holds the three x-shifts of
 //    a 1-channel tensor): the taps along x are channels,
 //    the box has no x halo, and a K step of 16 is two rows y (the tap pairs
@@ -49,6 +58,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <cfloat>
 
 #include "common.cuh"
 #include "conv.cuh"
@@ -64,15 +74,25 @@ constexpr int C3_THREADS = 64 + 32 * C3_EPI;
 constexpr int C3_MAX_STAGES = 8;
 constexpr int C3_MAX_CO = 128;
 constexpr uint32_t C3_SMEM = 224u * 1024u;
+constexpr int C3_REDO = 256;  // words of the bit field of tiles to do again
 constexpr int TX = 8, TY = 16;  // voxels of a tile along x and y
 
 struct C3Geom {
   int nx, ny, nz, nb, tiles_x, tiles_y, tiles_z, ntiles;
   int groups, stages;    // groups of 16 input channels
-  int K, CO, N, rb;      // input channels of w, channels per CTA, columns, rows of a weight tap
+  int K, CO, N, rb;      // input channels of w, channels per CTA (a multiple of 16), columns,
+                         // rows of a weight tap
   int late_w;            // the kernel before may have written the weights
   uint32_t wbytes, ncols;
 };
+
+// max of `top` and |v|, NaN if one is NaN
+__device__ __forceinline__ float max_abs(const float (&v)[16], float top) {
+#pragma unroll
+  for (int e = 0; e < 16; e++)
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(fabsf(v[e])));
+  return top;
+}
 
 template <int ZO, bool PACK>
 __global__ void __launch_bounds__(C3_THREADS, 1)
@@ -91,6 +111,7 @@ __global__ void __launch_bounds__(C3_THREADS, 1)
   __shared__ __align__(16) float sbias[C3_MAX_CO];
   __shared__ uint32_t tslot;
   __shared__ volatile int abort_flag;
+  __shared__ uint32_t redo[C3_REDO], redo_any;
   uint8_t* base = dsm + ((128u - (umma::smem_u32(dsm) & 127u)) & 127u);
   uint8_t* stages = base + g.wbytes;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -107,6 +128,7 @@ __global__ void __launch_bounds__(C3_THREADS, 1)
     }
     umma::mbar_init(&done, 1);
     abort_flag = 0;
+    redo_any = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -119,6 +141,7 @@ __global__ void __launch_bounds__(C3_THREADS, 1)
   if (g.late_w) pdl_wait();
   // ---- weights: [group][K step][chunk][row of rb][8 channels]; row = plane
   // * CO + co, plane p holding tap z = ZO + 1 - p where that is 0, 1 or 2
+  for (int c = threadIdx.x; c < C3_REDO; c += C3_THREADS) redo[c] = 0u;
   for (int c = threadIdx.x; c < C3_MAX_CO; c += C3_THREADS)
     sbias[c] = (ep.bias && c < g.CO && co0 + c < ep.Nout) ? ep.bias[co0 + c] : 0.0f;
   const int rows = G * TAPS * 2 * g.rb;
@@ -157,235 +180,278 @@ __global__ void __launch_bounds__(C3_THREADS, 1)
   const uint32_t tbase = tslot;
   const int my_tiles =
       (int)blockIdx.x < g.ntiles ? (g.ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  // a bit of `redo` stands for 2^rsh tiles
+  int rsh = 0;
+  while (((my_tiles - 1) >> rsh) >= 32 * C3_REDO) rsh++;
   bool timed_out = false;
   // a tile's place, stepped by gridDim.x tiles with carries
-  int tix = (int)blockIdx.x, sx_ = (int)gridDim.x;
-  int tiy = tix / g.tiles_x, sy_ = sx_ / g.tiles_x;
-  tix -= tiy * g.tiles_x, sx_ -= sy_ * g.tiles_x;
-  int tiz = tiy / g.tiles_y, sz_ = sy_ / g.tiles_y;
-  tiy -= tiz * g.tiles_y, sy_ -= sz_ * g.tiles_y;
-  int tib = tiz / g.tiles_z, sb_ = sz_ / g.tiles_z;
-  tiz -= tib * g.tiles_z, sz_ -= sb_ * g.tiles_z;
+  int tix, tiy, tiz, tib;
+  auto first_tile = [&] {
+    tix = (int)blockIdx.x;
+    tiy = tix / g.tiles_x, tix -= tiy * g.tiles_x;
+    tiz = tiy / g.tiles_y, tiy -= tiz * g.tiles_y;
+    tib = tiz / g.tiles_z, tiz -= tib * g.tiles_z;
+  };
+  int sx_ = (int)gridDim.x;
+  int sy_ = sx_ / g.tiles_x;
+  sx_ -= sy_ * g.tiles_x;
+  int sz_ = sy_ / g.tiles_y;
+  sy_ -= sz_ * g.tiles_y;
+  const int sb_ = sz_ / g.tiles_z;
+  sz_ -= sb_ * g.tiles_z;
   auto next_tile = [&] {
     tix += sx_, tiy += sy_, tiz += sz_, tib += sb_;
     if (tix >= g.tiles_x) tix -= g.tiles_x, tiy++;
     if (tiy >= g.tiles_y) tiy -= g.tiles_y, tiz++;
     if (tiz >= g.tiles_z) tiz -= g.tiles_z, tib++;
   };
-  if (warp == 0) {
-    // ---- loads
-    int s = 0, issued = 0;
-    uint32_t phase = 1u;
-    for (int jt = 0; jt < my_tiles && !timed_out; jt++) {
-      for (int grp = 0; grp < G; grp++) {
+  // what each role carries from tile to tile: the tiles it has taken, the loads
+  // issued, the stage and its phase
+  int it = 0, issued = 0, s = 0;
+  uint32_t phase = warp == 0 ? 1u : 0u;
+  // pass 0: every tile; pass 1: those with sums that are not finite, again
+  for (int pass = 0; pass < (ZO > 1 ? 2 : 1); pass++) {
+    if (pass == 1 && (__syncthreads_or(timed_out) || !redo_any)) break;
+    first_tile();
+    auto skip = [&](int jt) {
+      return pass == 1 && !((redo[jt >> rsh >> 5] >> ((jt >> rsh) & 31)) & 1u);
+    };
+    if (warp == 0) {
+      // ---- loads
+      for (int jt = 0; jt < my_tiles && !timed_out; jt++, next_tile()) {
+        if (skip(jt)) continue;
+        for (int grp = 0; grp < G; grp++) {
+          if (abort_flag) break;
+          if (issued >= S && !umma::mbar_wait_warp(&empty[s], phase)) {
+            timed_out = true;
+            break;
+          }
+          // a box per plane and chunk, each from its own lane
+          if (lane == 0) umma::mbar_expect_tx(&full[s], CHUNKS * ZI * BOX);
+          __syncwarp();
+          if (lane < CHUNKS * ZI) {
+            const int ch = lane / ZI, zi = lane - ch * ZI;
+            umma::tma_load_5d(stages + (size_t)s * STAGE + (uint32_t)lane * PLANE, &tx,
+                              (tix * TX - (PACK ? 0 : 1)) * 8, tiy * TY - 1, tiz * ZO - 1 + zi,
+                              PACK ? 0 : grp * 2 + ch, tib, &full[s]);
+          }
+          issued++;
+          if (++s == S) s = 0, phase ^= 1u;
+        }
         if (abort_flag) break;
-        if (issued >= S && !umma::mbar_wait_warp(&empty[s], phase)) {
+      }
+      if (timed_out) abort_flag = 1;
+    } else if (warp == 1) {
+      // ---- MMAs.  Descriptors: the high word holds the stride between core
+      // matrices of 8 rows, the low word the K halves' distance and the address
+      // in 16-byte units.
+      const uint32_t idesc = umma::idesc_bf16(128, g.N);
+      const uint32_t hi_a = (ROW >> 4) | (1u << 14), hi_b = (128u >> 4) | (1u << 14);
+      const uint32_t lo_a = ((PACK ? ROW : CHUNK) >> 4) << 16;
+      const uint32_t step = 2u * (uint32_t)g.rb;  // one K step of weights
+      const uint32_t co16 = (uint32_t)g.CO;       // one plane of weight rows
+      const uint32_t wb = (umma::smem_u32(base) >> 4) | ((uint32_t)g.rb << 16);
+      for (int jt = 0; jt < my_tiles && !timed_out; jt++) {
+        if (skip(jt)) continue;
+        const int a = it & 1;
+        if (abort_flag) break;
+        if (it >= 2 && !umma::mbar_wait_warp(&acce[a], ((it >> 1) - 1) & 1)) {
           timed_out = true;
           break;
         }
-        // a box per plane and chunk, each from its own lane
-        if (lane == 0) umma::mbar_expect_tx(&full[s], CHUNKS * ZI * BOX);
-        __syncwarp();
-        if (lane < CHUNKS * ZI) {
-          const int ch = lane / ZI, zi = lane - ch * ZI;
-          umma::tma_load_5d(stages + (size_t)s * STAGE + (uint32_t)lane * PLANE, &tx,
-                            (tix * TX - (PACK ? 0 : 1)) * 8, tiy * TY - 1, tiz * ZO - 1 + zi,
-                            PACK ? 0 : grp * 2 + ch, tib, &full[s]);
+        const uint32_t dt = tbase + (uint32_t)(a * g.N);
+        for (int grp = 0; grp < G; grp++) {
+          if (abort_flag) break;
+          if (!umma::mbar_wait_warp(&full[s], phase)) {
+            timed_out = true;
+            break;
+          }
+          umma::fence_after();
+          uint32_t da = ((umma::smem_u32(stages) + (uint32_t)s * STAGE) >> 4) | lo_a;
+          uint32_t db = wb + (uint32_t)(grp * TAPS) * step + (uint32_t)(ZO + 1) * co16;
+          // the MMAs of one input plane at d_, into the columns at c_
+          auto plane = [&](uint32_t c_, uint32_t d_, uint32_t w_, uint32_t id, uint32_t acc) {
+            if (umma::elect_one()) {
+#pragma unroll
+              for (int t = 0; t < TAPS; t++) {
+                const uint32_t off = PACK ? (uint32_t)t * (ROW >> 4)
+                                          : (uint32_t)(t / 3) * (ROW >> 4) + (uint32_t)(t % 3);
+                umma::mma_bf16(c_, ((uint64_t)hi_a << 32) | (d_ + off),
+                               ((uint64_t)hi_b << 32) | (w_ + t * step), id, t ? 1u : acc);
+              }
+            }
+          };
+          if (pass == 0) {
+#pragma unroll 1
+            for (int zi = 0; zi < ZI; zi++) {
+              plane(dt, da, db, idesc, grp > 0 || zi > 0 ? 1u : 0u);
+              da += PLANE >> 4;
+              db -= co16;
+            }
+          } else {
+#pragma unroll 1
+            for (int zo = 0; zo < ZO; zo++)
+#pragma unroll 1
+              for (int tz = 0; tz < 3; tz++)
+                plane(dt + (uint32_t)zo * co16, da + (uint32_t)(zo + tz) * (PLANE >> 4),
+                      db - (uint32_t)tz * co16, umma::idesc_bf16(128, g.CO),
+                      grp > 0 || tz > 0 ? 1u : 0u);
+          }
+          if (umma::elect_one()) umma::mma_commit(&empty[s]);
+          if (++s == S) s = 0, phase ^= 1u;
         }
-        issued++;
-        if (++s == S) s = 0, phase ^= 1u;
+        if (timed_out || abort_flag) break;
+        if (umma::elect_one()) umma::mma_commit(&accf[a]);
+        it++;
       }
-      if (abort_flag) break;
-      next_tile();
+      if (timed_out) abort_flag = 1;
+    } else {
+      // ---- epilogue: lane = row of D = voxel (x = m % 8, y = m / 8); a column
+      // is (zo, channel).  Two warps share the lanes of a quarter of D and take
+      // its pairs of 16-column groups in turn.
+      const int q = warp & 3, m = q * 32 + lane, half = (warp - 2) >> 2;
+      // whole 8-channel chunks, 16-byte accesses of the output and the mask
+      const bool planes = ep.out_bf16 && !(ep.Nout & 7) &&
+                          !((reinterpret_cast<uintptr_t>(ep.out_bf16) |
+                             reinterpret_cast<uintptr_t>(ep.mask)) & 15);
+      const int gpz = g.CO >> 4;  // 16-column groups per output plane
+      for (int jt = 0; jt < my_tiles; jt++, next_tile()) {
+        if (skip(jt)) continue;
+        const int a = it & 1;
+        if (!umma::mbar_wait_warp(&accf[a], (it >> 1) & 1)) {
+          timed_out = true;
+          abort_flag = 1;
+          break;
+        }
+        umma::fence_after();
+        const int x = tix * TX + (m & 7), y = tiy * TY + (m >> 3), z0 = tiz * ZO;
+        const bool in = x < g.nx && y < g.ny;
+        const size_t v0 = (((size_t)tib * g.nz + z0) * g.ny + y) * g.nx + x;
+        const size_t zs = (size_t)g.ny * g.nx;
+        const uint32_t ta = tbase + (uint32_t)(a * g.N) + ((uint32_t)(q * 32) << 16);
+        float top = 0.0f;  // the largest |sum|; NaN stays
+        if (planes) {
+          const int ng = g.N >> 4;
+          for (int k0 = 2 * half; k0 < ng; k0 += 4) {
+            // a pair of groups, their four masks loaded ahead
+            size_t o[2];
+            int c[2];
+            bool own[2][2];
+            uint4 mk[2][2];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+              int zo, cg;
+              if constexpr (ZO == 1) {
+                zo = k0 + k < gpz ? 0 : ZO;
+                cg = k0 + k;
+              } else {
+                zo = gpz == 1 ? k0 + k : (k0 + k) / gpz;
+                cg = k0 + k - zo * gpz;
+              }
+              c[k] = cg * 16;
+              o[k] = (size_t)((co0 + c[k]) >> 3) * ep.V + v0 + (size_t)zo * zs;
+#pragma unroll
+              for (int h = 0; h < 2; h++) {
+                own[k][h] = in && k0 + k < ng && zo < ZO && z0 + zo < g.nz &&
+                            co0 + c[k] + 8 * h < ep.Nout;
+                if (ep.mask && own[k][h])
+                  mk[k][h] = __ldg(reinterpret_cast<const uint4*>(ep.mask) + o[k] +
+                                   (size_t)h * ep.V);
+              }
+            }
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+              if (k0 + k >= ng) break;
+              float v[16];
+              umma::tmem_ld16(ta + (uint32_t)((k0 + k) * 16), v);
+              if (ZO > 1) top = max_abs(v, top);
+#pragma unroll
+              for (int h = 0; h < 2; h++) {
+                if (!own[k][h]) continue;
+                const float4 b0 = *reinterpret_cast<const float4*>(sbias + c[k] + 8 * h),
+                             b1 = *reinterpret_cast<const float4*>(sbias + c[k] + 8 * h + 4);
+                float r[8] = {v[8 * h] + b0.x,     v[8 * h + 1] + b0.y, v[8 * h + 2] + b0.z,
+                              v[8 * h + 3] + b0.w, v[8 * h + 4] + b1.x, v[8 * h + 5] + b1.y,
+                              v[8 * h + 6] + b1.z, v[8 * h + 7] + b1.w};
+                if (ep.relu) {
+#pragma unroll
+                  for (int e = 0; e < 8; e++) r[e] = fmaxf(r[e], 0.0f);
+                }
+                uint4 u;
+                __nv_bfloat162* ub = reinterpret_cast<__nv_bfloat162*>(&u);
+#pragma unroll
+                for (int e = 0; e < 4; e++) ub[e] = __floats2bfloat162_rn(r[2 * e], r[2 * e + 1]);
+                if (ep.mask) {
+                  // keep a BF16 half only where the mask half is > 0
+                  const uint32_t* mw = reinterpret_cast<const uint32_t*>(&mk[k][h]);
+                  uint32_t* uw = reinterpret_cast<uint32_t*>(&u);
+#pragma unroll
+                  for (int e = 0; e < 4; e++) {
+                    const float lo = __uint_as_float(mw[e] << 16),
+                                hi = __uint_as_float(mw[e] & 0xFFFF0000u);
+                    uw[e] &= (lo > 0.0f ? 0x0000FFFFu : 0u) | (hi > 0.0f ? 0xFFFF0000u : 0u);
+                  }
+                }
+                if (ep.up) {
+                  const int z = 2 * (z0 + (ZO == 1 ? 0 : (k0 + k) / gpz));
+                  uint4* q8 = reinterpret_cast<uint4*>(ep.out_bf16) +
+                              (size_t)(((co0 + c[k]) >> 3) + h) * ep.fV;
+#pragma unroll
+                  for (int j = 0; j < 4; j++) {
+                    const int fz = z + (j >> 1), fy = 2 * y + (j & 1);
+                    if (fz >= ep.fz || fy >= ep.fy) continue;
+                    uint4* row = q8 + (((size_t)tib * ep.fz + fz) * ep.fy + fy) * ep.fx + 2 * x;
+                    row[0] = u;
+                    if (2 * x + 1 < ep.fx) row[1] = u;
+                  }
+                } else {
+                  reinterpret_cast<uint4*>(ep.out_bf16)[o[k] + (size_t)h * ep.V] = u;
+                }
+              }
+            }
+          }
+        } else {
+          for (int col = 16 * half; col < g.N; col += 32) {
+            float v[16];
+            umma::tmem_ld16(ta + (uint32_t)col, v);
+            if (ZO > 1) top = max_abs(v, top);
+            const int zo = col / g.CO, c0 = col - zo * g.CO;
+            if (!in || z0 + zo >= g.nz) continue;
+            const size_t vox = v0 + (size_t)zo * zs;
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+              const int c = c0 + k, co = co0 + c;
+              if (co >= ep.Nout) break;
+              float val = v[k] + sbias[c];
+              if (ep.relu) val = fmaxf(val, 0.0f);
+              if (ep.mask && !(__bfloat162float(ep.mask[act_off(vox, co, ep.Nout, ep.V)]) > 0.0f))
+                val = 0.0f;
+              if (ep.out_f32) ep.out_f32[vox * ep.Nout + co] = val;
+              else ep.out_bf16[act_off(vox, co, ep.Nout, ep.V)] = __float2bfloat16_rn(val);
+            }
+          }
+        }
+        if (ZO > 1 && pass == 0 && __any_sync(0xffffffffu, !(top <= FLT_MAX)) && lane == 0) {
+          atomicOr(&redo[jt >> rsh >> 5], 1u << ((jt >> rsh) & 31));
+          redo_any = 1u;
+        }
+        umma::fence_before();
+        __syncwarp();
+        if (lane == 0)
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smem_u32(&acce[a]))
+                       : "memory");
+        it++;
+      }
     }
-    if (timed_out) abort_flag = 1;
+  }
+  if (warp == 0) {
     // every issued copy lands before the CTA may exit
     for (int q = issued > S ? issued - S : 0; q < issued; q++)
       if (!umma::mbar_wait_warp(&full[q % S], (q / S) & 1)) timed_out = true;
   } else if (warp == 1) {
-    // ---- MMAs.  Descriptors: the high word holds the stride between core
-    // matrices of 8 rows, the low word the K halves' distance and the address
-    // in 16-byte units.
-    const uint32_t idesc = umma::idesc_bf16(128, g.N);
-    const uint32_t hi_a = (ROW >> 4) | (1u << 14), hi_b = (128u >> 4) | (1u << 14);
-    const uint32_t lo_a = ((PACK ? ROW : CHUNK) >> 4) << 16;
-    const uint32_t step = 2u * (uint32_t)g.rb;  // one K step of weights
-    const uint32_t co16 = (uint32_t)g.CO;       // one plane of weight rows
-    const uint32_t wb = (umma::smem_u32(base) >> 4) | ((uint32_t)g.rb << 16);
-    int s = 0;
-    uint32_t phase = 0u;
-    for (int jt = 0; jt < my_tiles && !timed_out; jt++) {
-      const int a = jt & 1;
-      if (abort_flag) break;
-      if (jt >= 2 && !umma::mbar_wait_warp(&acce[a], ((jt >> 1) - 1) & 1)) {
-        timed_out = true;
-        break;
-      }
-      const uint32_t dt = tbase + (uint32_t)(a * g.N);
-      for (int grp = 0; grp < G; grp++) {
-        if (abort_flag) break;
-        if (!umma::mbar_wait_warp(&full[s], phase)) {
-          timed_out = true;
-          break;
-        }
-        umma::fence_after();
-        uint32_t da = ((umma::smem_u32(stages) + (uint32_t)s * STAGE) >> 4) | lo_a;
-        uint32_t db = wb + (uint32_t)(grp * TAPS) * step + (uint32_t)(ZO + 1) * co16;
-        uint32_t acc = grp > 0 ? 1u : 0u;
-#pragma unroll 1
-        for (int zi = 0; zi < ZI; zi++) {
-          if (umma::elect_one()) {
-#pragma unroll
-            for (int t = 0; t < TAPS; t++) {
-              const uint32_t off = PACK ? (uint32_t)t * (ROW >> 4)
-                                        : (uint32_t)(t / 3) * (ROW >> 4) + (uint32_t)(t % 3);
-              umma::mma_bf16(dt, ((uint64_t)hi_a << 32) | (da + off),
-                             ((uint64_t)hi_b << 32) | (db + t * step), idesc, t ? 1u : acc);
-            }
-          }
-          acc = 1u;
-          da += PLANE >> 4;
-          db -= co16;
-        }
-        if (umma::elect_one()) umma::mma_commit(&empty[s]);
-        if (++s == S) s = 0, phase ^= 1u;
-      }
-      if (timed_out || abort_flag) break;
-      if (umma::elect_one()) umma::mma_commit(&accf[a]);
-    }
-    if (timed_out) abort_flag = 1;
     // every MMA issued has finished before the TMEM is freed
     if (umma::elect_one()) umma::mma_commit(&done);
     if (!umma::mbar_wait_warp(&done, 0)) timed_out = true;
-  } else {
-    // ---- epilogue: lane = row of D = voxel (x = m % 8, y = m / 8); a column
-    // is (zo, channel).  Two warps share the lanes of a quarter of D and take
-    // its pairs of 16-column groups in turn.
-    const int q = warp & 3, m = q * 32 + lane, half = (warp - 2) >> 2;
-    // whole 8-channel chunks, 16-byte accesses of the output and the mask
-    const bool planes = ep.out_bf16 && !(ep.Nout & 7) && !(g.CO & 15) &&
-                        !((reinterpret_cast<uintptr_t>(ep.out_bf16) |
-                           reinterpret_cast<uintptr_t>(ep.mask)) & 15);
-    const int gpz = g.CO >> 4;  // 16-column groups per output plane
-    for (int jt = 0; jt < my_tiles; jt++) {
-      const int a = jt & 1;
-      if (!umma::mbar_wait_warp(&accf[a], (jt >> 1) & 1)) {
-        timed_out = true;
-        abort_flag = 1;
-        break;
-      }
-      umma::fence_after();
-      const int x = tix * TX + (m & 7), y = tiy * TY + (m >> 3), z0 = tiz * ZO;
-      const bool in = x < g.nx && y < g.ny;
-      const size_t v0 = (((size_t)tib * g.nz + z0) * g.ny + y) * g.nx + x;
-      const size_t zs = (size_t)g.ny * g.nx;
-      const uint32_t ta = tbase + (uint32_t)(a * g.N) + ((uint32_t)(q * 32) << 16);
-      if (planes) {
-        const int ng = g.N >> 4;
-        for (int k0 = 2 * half; k0 < ng; k0 += 4) {
-          // a pair of groups, their four masks loaded ahead
-          size_t o[2];
-          int c[2];
-          bool own[2][2];
-          uint4 mk[2][2];
-#pragma unroll
-          for (int k = 0; k < 2; k++) {
-            int zo, cg;
-            if constexpr (ZO == 1) {
-              zo = k0 + k < gpz ? 0 : ZO;
-              cg = k0 + k;
-            } else {
-              zo = gpz == 1 ? k0 + k : (k0 + k) / gpz;
-              cg = k0 + k - zo * gpz;
-            }
-            c[k] = cg * 16;
-            o[k] = (size_t)((co0 + c[k]) >> 3) * ep.V + v0 + (size_t)zo * zs;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-              own[k][h] = in && k0 + k < ng && zo < ZO && z0 + zo < g.nz &&
-                          co0 + c[k] + 8 * h < ep.Nout;
-              if (ep.mask && own[k][h])
-                mk[k][h] = __ldg(reinterpret_cast<const uint4*>(ep.mask) + o[k] +
-                                 (size_t)h * ep.V);
-            }
-          }
-#pragma unroll
-          for (int k = 0; k < 2; k++) {
-            if (k0 + k >= ng) break;
-            float v[16];
-            umma::tmem_ld16(ta + (uint32_t)((k0 + k) * 16), v);
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-              if (!own[k][h]) continue;
-              const float4 b0 = *reinterpret_cast<const float4*>(sbias + c[k] + 8 * h),
-                           b1 = *reinterpret_cast<const float4*>(sbias + c[k] + 8 * h + 4);
-              float r[8] = {v[8 * h] + b0.x,     v[8 * h + 1] + b0.y, v[8 * h + 2] + b0.z,
-                            v[8 * h + 3] + b0.w, v[8 * h + 4] + b1.x, v[8 * h + 5] + b1.y,
-                            v[8 * h + 6] + b1.z, v[8 * h + 7] + b1.w};
-              if (ep.relu) {
-#pragma unroll
-                for (int e = 0; e < 8; e++) r[e] = fmaxf(r[e], 0.0f);
-              }
-              uint4 u;
-              __nv_bfloat162* ub = reinterpret_cast<__nv_bfloat162*>(&u);
-#pragma unroll
-              for (int e = 0; e < 4; e++) ub[e] = __floats2bfloat162_rn(r[2 * e], r[2 * e + 1]);
-              if (ep.mask) {
-                // keep a BF16 half only where the mask half is > 0
-                const uint32_t* mw = reinterpret_cast<const uint32_t*>(&mk[k][h]);
-                uint32_t* uw = reinterpret_cast<uint32_t*>(&u);
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                  const float lo = __uint_as_float(mw[e] << 16),
-                              hi = __uint_as_float(mw[e] & 0xFFFF0000u);
-                  uw[e] &= (lo > 0.0f ? 0x0000FFFFu : 0u) | (hi > 0.0f ? 0xFFFF0000u : 0u);
-                }
-              }
-              if (ep.up) {
-                const int z = 2 * (z0 + (ZO == 1 ? 0 : (k0 + k) / gpz));
-                uint4* q8 = reinterpret_cast<uint4*>(ep.out_bf16) +
-                            (size_t)(((co0 + c[k]) >> 3) + h) * ep.fV;
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                  const int fz = z + (j >> 1), fy = 2 * y + (j & 1);
-                  if (fz >= ep.fz || fy >= ep.fy) continue;
-                  uint4* row = q8 + (((size_t)tib * ep.fz + fz) * ep.fy + fy) * ep.fx + 2 * x;
-                  row[0] = u;
-                  if (2 * x + 1 < ep.fx) row[1] = u;
-                }
-              } else {
-                reinterpret_cast<uint4*>(ep.out_bf16)[o[k] + (size_t)h * ep.V] = u;
-              }
-            }
-          }
-        }
-      } else {
-        for (int col = 16 * half; col < g.N; col += 32) {
-          float v[16];
-          umma::tmem_ld16(ta + (uint32_t)col, v);
-          if (!in) continue;
-#pragma unroll
-          for (int k = 0; k < 16; k++) {
-            const int cc = col + k, zo = g.CO == 1 ? cc : cc / g.CO, c = cc - zo * g.CO,
-                      co = co0 + c;
-            if (zo >= ZO || z0 + zo >= g.nz || co >= ep.Nout) continue;
-            const size_t vox = v0 + (size_t)zo * zs;
-            float val = v[k] + sbias[c];
-            if (ep.relu) val = fmaxf(val, 0.0f);
-            if (ep.mask && !(__bfloat162float(ep.mask[act_off(vox, co, ep.Nout, ep.V)]) > 0.0f))
-              val = 0.0f;
-            if (ep.out_f32) ep.out_f32[vox * ep.Nout + co] = val;
-            else ep.out_bf16[act_off(vox, co, ep.Nout, ep.V)] = __float2bfloat16_rn(val);
-          }
-        }
-      }
-      umma::fence_before();
-      __syncwarp();
-      if (lane == 0)
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::smem_u32(&acce[a]))
-                     : "memory");
-      next_tile();
-    }
   }
   if (timed_out && lane == 0) atomicExch(err, 1);
   umma::fence_before();
@@ -413,16 +479,19 @@ struct C3Plan {
 // of tiles times a tile's MMAs, plus the weights each CTA writes first (about
 // 1 cycle per 16-byte row and thread).  Tall tiles pay while there are waves
 // of them; a small volume takes flat ones so that every SM has a tile.
-C3Plan c3_plan(int nx, int ny, int nz, int nb, int groups, int N_out, bool pack, int nsm) {
+// flat: one plane per tile, for an output that overwrites its mask (a tile that
+// is done again reads the mask again).
+C3Plan c3_plan(int nx, int ny, int nz, int nb, int groups, int N_out, bool pack, bool flat,
+               int nsm) {
   C3Plan best;
   const int taps = pack ? 2 : 9;
   for (int zo : {1, 2, 4, 8}) {
-    if (zo > 1 && zo / 2 >= nz) continue;
+    if (zo > 1 && (flat || zo / 2 >= nz)) continue;
     for (int split = 1; split <= (N_out + 15) / 16; split++) {
-      const int co = split == 1 ? N_out : ((N_out + split - 1) / split + 15) / 16 * 16;
+      const int co = ((N_out + split - 1) / split + 15) / 16 * 16;
       if (split > 1 && (co * (split - 1) >= N_out)) continue;
       if (co > C3_MAX_CO) continue;
-      const int N = (zo * co + 15) / 16 * 16;
+      const int N = zo * co;
       if (N > 256) continue;
       const long rb = (long)(zo + 1) * co + N;
       const long wbytes = ((long)groups * taps * 2 * rb * 16 + 127) / 128 * 128;
@@ -472,11 +541,15 @@ cudaError_t conv3_tma(const bf16* x, int K, bool pack, int nx, int ny, int nz, i
   g.K = K;
   g.late_w = old_weights ? 0 : 1;
   g.groups = pack ? 1 : K / 16;
-  const C3Plan pl = c3_plan(nx, ny, nz, nb, g.groups, N, pack, nsm);
+  // the bytes of a BF16 or FP32 output and of its mask
+  const size_t elems = (size_t)nx * ny * nz * nb * N;
+  const char *y0 = y_f32 ? (const char*)y_f32 : (const char*)y_bf16, *m0 = (const char*)mask;
+  const bool flat = mask && y0 < m0 + elems * 2 && m0 < y0 + elems * (y_f32 ? 4 : 2);
+  const C3Plan pl = c3_plan(nx, ny, nz, nb, g.groups, N, pack, flat, nsm);
   if (!pl.zo) return cudaErrorInvalidValue;
   const int taps = pack ? 2 : 9, px = pack ? TX : TX + 2;
   g.CO = pl.co;
-  g.N = (pl.zo * pl.co + 15) / 16 * 16;
+  g.N = pl.zo * pl.co;
   g.rb = (pl.zo + 1) * pl.co + g.N;
   g.stages = pl.stages;
   g.wbytes = ((uint32_t)(g.groups * taps * 2 * g.rb) * 16u + 127u) & ~127u;

@@ -214,3 +214,74 @@ def test_narrow_layers_sum_in_fp32_order(lib, C, Cout, dims):
                                 None)
     assert rc == 0, lib.pyro_last_error()
     assert torch.equal(y.permute(0, 4, 1, 2, 3), acc)
+
+
+def _bad_voxels(x, at, channel):
+    """x with NaN, Inf and -Inf at three voxels, and the mask of the voxels
+    within one cell of them."""
+    bad, near = x.clone(), torch.zeros(x.shape[2:], dtype=torch.bool, device=x.device)
+    for (z, y, xx), v in zip(at, (float("nan"), float("inf"), -float("inf"))):
+        bad[0, channel, z, y, xx] = v
+        near[max(z - 1, 0):z + 2, max(y - 1, 0):y + 2, max(xx - 1, 0):xx + 2] = True
+    return bad, near
+
+
+@pytest.mark.parametrize("C,Cout,dims", [(16, 16, (40, 100, 90)),  # four planes per tile
+                                         (48, 16, (40, 100, 90)),
+                                         (16, 48, (40, 100, 90)),  # two
+                                         (32, 4, (41, 65, 40)),    # columns padded to 16
+                                         (16, 16, (3, 17, 9))])    # a plane per tile
+@pytest.mark.parametrize("relu", [0, 1])
+def test_forward_not_finite_stays_local(lib, C, Cout, dims, relu):
+    """A voxel that is not finite reaches the outputs of its 27 neighbours, and
+    every other output keeps its bits."""
+    nz, ny, nx = dims
+    x, w, b = _tensors(1, C, nz, ny, nx, Cout, 31)
+    at = [(nz // 2, ny // 3, nx // 2), (nz - 1, ny - 1, 0), (0, ny // 2, nx - 1)]
+    bad, near = _bad_voxels(x, at, C - 3)
+    wk = _wk(w)
+    for f32 in (1, 0):
+        out = []
+        for t in (x, bad):
+            y = torch.full((nz * ny * nx * Cout,), 7.0,
+                           dtype=torch.float32 if f32 else torch.bfloat16, device="cuda")
+            tc = _cl(t)
+            rc = lib.pyro_conv3_forward(ptr(tc), C, nx, ny, nz, 1, ptr(wk), Cout, ptr(b), relu,
+                                        ptr(y), f32, None)
+            assert rc == 0, lib.pyro_last_error()
+            if f32 or Cout % 8:
+                out.append(y.view(nz, ny, nx, Cout))
+            else:
+                out.append(y.view(Cout // 8, nz, ny, nx, 8).permute(1, 2, 3, 0, 4)
+                           .reshape(nz, ny, nx, Cout))
+        assert torch.equal(out[1][~near], out[0][~near])
+        assert relu or not torch.isfinite(out[1][near]).any()
+
+
+@pytest.mark.parametrize("Cin,Cout,dims", [(16, 16, (40, 100, 90)), (48, 16, (40, 100, 90)),
+                                           (16, 32, (21, 65, 40))])
+def test_backward_data_not_finite_stays_local(lib, Cin, Cout, dims):
+    """The same of the data gradient, masked, into a tensor of its own and over
+    the mask."""
+    nz, ny, nx = dims
+    dy, _, _ = _tensors(1, Cout, nz, ny, nx, 1, 32)
+    act, w, _ = _tensors(1, Cin, nz, ny, nx, Cout, 33)
+    at = [(nz // 2, ny // 3, nx // 2), (nz - 1, ny - 1, 0), (0, ny // 2, nx - 1)]
+    bad, near = _bad_voxels(dy, at, 5)
+    wk, actc = _wk(w), _cl(act)
+    out = []
+    for t, inplace in ((dy, False), (bad, False), (bad, True)):
+        tc, ac = _cl(t), actc.clone()
+        dx = ac if inplace else torch.full_like(ac, 7.0)
+        rc = lib.pyro_conv3_backward_data(ptr(tc), Cout, nx, ny, nz, 1, ptr(wk), Cin, ptr(ac),
+                                          ptr(dx), 0, None)
+        assert rc == 0, lib.pyro_last_error()
+        out.append(dx.view(Cin // 8, nz, ny, nx, 8).permute(1, 2, 3, 0, 4)
+                   .reshape(nz, ny, nx, Cin))
+    on = act[0].permute(1, 2, 3, 0) > 0
+    far = ~near
+    assert torch.equal(out[1][far], out[0][far])
+    assert torch.equal(out[2][far], out[0][far])
+    for o in out[1:]:
+        assert not torch.isfinite(o[near][on[near]]).any()
+        assert (o[near][~on[near]] == 0).all()
