@@ -73,7 +73,11 @@ __device__ __forceinline__ void st_bf(uint8_t* s, uint32_t off, bf16 v) {
 
 template <int N, class Load, class Epi>
 __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(Load ld, Epi ep, int ksteps_total,
-                                                       int ksteps_per_cta, int* err) {
+                                                       int ksteps_per_cta, int* err,
+                                                       const int* only_if) {
+  pdl_trigger();
+  pdl_wait();
+  if (only_if && *only_if == 0) return;
   constexpr int NCOLS = N <= 32 ? 32 : (N <= 64 ? 64 : 128);
   __shared__ __align__(1024) uint8_t sA[2][128 * 32];
   __shared__ __align__(1024) uint8_t sB[2][N * 32];
@@ -261,21 +265,21 @@ struct WgradEpi {
 
 template <int N, class Load, class Epi>
 cudaError_t gemm_launch(dim3 grid, const Load& ld, const Epi& ep, int ksteps_total,
-                        int ksteps_per_cta, int* err, cudaStream_t st) {
-  k_gemm<N, Load, Epi><<<grid, GEMM_THREADS, 0, st>>>(ld, ep, ksteps_total, ksteps_per_cta, err);
-  return cudaGetLastError();
+                        int ksteps_per_cta, int* err, cudaStream_t st, const int* only_if) {
+  return launch_pdl(k_gemm<N, Load, Epi>, grid, dim3(GEMM_THREADS), 0, st, ld, ep, ksteps_total,
+                    ksteps_per_cta, err, only_if);
 }
 
 template <class Load, class Epi>
 cudaError_t gemm_dispatch(int npad, dim3 grid, const Load& ld, const Epi& ep, int kt, int kpc,
-                          int* err, cudaStream_t st) {
+                          int* err, cudaStream_t st, const int* only_if = nullptr) {
   switch (npad) {
-    case 16: return gemm_launch<16>(grid, ld, ep, kt, kpc, err, st);
-    case 32: return gemm_launch<32>(grid, ld, ep, kt, kpc, err, st);
-    case 48: return gemm_launch<48>(grid, ld, ep, kt, kpc, err, st);
-    case 64: return gemm_launch<64>(grid, ld, ep, kt, kpc, err, st);
-    case 96: return gemm_launch<96>(grid, ld, ep, kt, kpc, err, st);
-    case 128: return gemm_launch<128>(grid, ld, ep, kt, kpc, err, st);
+    case 16: return gemm_launch<16>(grid, ld, ep, kt, kpc, err, st, only_if);
+    case 32: return gemm_launch<32>(grid, ld, ep, kt, kpc, err, st, only_if);
+    case 48: return gemm_launch<48>(grid, ld, ep, kt, kpc, err, st, only_if);
+    case 64: return gemm_launch<64>(grid, ld, ep, kt, kpc, err, st, only_if);
+    case 96: return gemm_launch<96>(grid, ld, ep, kt, kpc, err, st, only_if);
+    case 128: return gemm_launch<128>(grid, ld, ep, kt, kpc, err, st, only_if);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -420,6 +424,14 @@ __global__ void k_wprep(const bf16* __restrict__ w, int Cout, int Cin, int backw
   }
 }
 
+// dw += s, nothing when *bad is set
+__global__ void __launch_bounds__(256) k_add_unless(const float* __restrict__ s, int n,
+                                                    const int* __restrict__ bad,
+                                                    float* __restrict__ dw) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i < n && !*bad) dw[i] += s[i];
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   static std::once_flag once;
@@ -468,18 +480,15 @@ cudaError_t conv3_backward_data(const bf16* dy, int Cout, int nx, int ny, int nz
   return gemm_dispatch(npad, grid, ld, ep, ksteps, ksteps, err, st);
 }
 
-// dw[co][tap][ci] += sum_voxels dy[v][co] x[v + tap][ci]  (dw FP32, zeroed
-// by the caller).
-cudaError_t conv3_backward_weight(const bf16* x, int Cin, const bf16* dy, int Cout, int nx,
-                                  int ny, int nz, int nb, float* dw, int* err, cudaStream_t st) {
-  // the boxes need 16-byte aligned tensors; others are gathered
-  const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy);
-  if (conv3_wgrad_fits(Cin, Cout) && at % 16 == 0)
-    return conv3_wgrad_tma(x, Cin, dy, Cout, 0, nx, ny, nz, nb, dw, err, st);
+// dw[co][tap][ci] += sum_voxels dy[v][co] x[v + tap][ci]  (dw FP32).
+cudaError_t conv3_wgrad_gather(const bf16* x, int Cin, const bf16* dy, int Cout, int nx, int ny,
+                               int nz, int nb, float* dw, int* err, const int* only_if,
+                               cudaStream_t st) {
   Vol g{nx, ny, nz, nb};
   int V = nx * ny * nz * nb;
   int M = 27 * Cin;
   int npad = pad16(Cout);
+  if (only_if && npad > 64) npad = npad > 96 ? 128 : 96;  // behind the boxes, which take 80 and 112
   int ksteps = (V + 15) / 16;
   int mt = (M + 127) / 128;
   // split K so that the grid covers the GPU a few times over
@@ -489,9 +498,8 @@ cudaError_t conv3_backward_weight(const bf16* x, int Cin, const bf16* dy, int Co
   WgradLoad ld{x, dy, g, Cin, Cout, npad};
   WgradEpi ep{dw, M, Cout};
   dim3 grid(mt, splits, 1);
-  return gemm_dispatch(npad, grid, ld, ep, ksteps, kpc, err, st);
+  return gemm_dispatch(npad, grid, ld, ep, ksteps, kpc, err, st, only_if);
 }
-
 
 // Direct convolution for the shapes k_conv_direct covers (2 -> 16 and
 // 16 -> 1 channels); cudaErrorInvalidValue for others.
@@ -616,12 +624,29 @@ int pyro_conv3_backward_weight(const void* x, int Cin, const void* dy, int Cout,
   PYRO_REQUIRE(x && dy && dw, "pyro_conv3_backward_weight: null buffer");
   PYRO_REQUIRE(conv_dims_ok(nx, ny, nz, nb) && chan_ok(Cin) && chan_ok(Cout),
                "pyro_conv3_backward_weight: invalid sizes");
-  DevBuf err;
-  int rc = err.alloc(4);
+  // the boxes need 16-byte aligned tensors; others are gathered, and so is a
+  // gradient with sums that are not finite
+  const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy);
+  const bool boxes = conv3_wgrad_fits(Cin, Cout) && at % 16 == 0;
+  const int n = Cout * 27 * Cin;
+  DevBuf err;  // the error and bad flags, then the boxes' sums
+  int rc = err.alloc(16 + (boxes ? (size_t)n * 4 : 0));
   if (rc != PYRO_OK) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  cudaError_t e = conv3_backward_weight((const bf16*)x, Cin, (const bf16*)dy, Cout, nx, ny, nz,
-                                        nb, dw, err.as<int>(), st);
+  int *E = err.as<int>(), *bad = boxes ? E + 1 : nullptr;
+  cudaError_t e = cudaSuccess;
+  if (boxes) {
+    float* sums = err.as<float>() + 4;
+    e = conv3_wgrad_tma((const bf16*)x, Cin, (const bf16*)dy, Cout, 0, nx, ny, nz, nb, sums, E,
+                        bad, st);
+    if (e == cudaSuccess) {
+      k_add_unless<<<(n + 255) / 256, 256, 0, st>>>(sums, n, bad, dw);
+      e = cudaGetLastError();
+    }
+  }
+  if (e == cudaSuccess)
+    e = conv3_wgrad_gather((const bf16*)x, Cin, (const bf16*)dy, Cout, nx, ny, nz, nb, dw, E, bad,
+                           st);
   return finish(e, err, st, "pyro_conv3_backward_weight");
 }
 

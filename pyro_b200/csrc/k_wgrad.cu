@@ -28,6 +28,12 @@
 // 16 47 ms -> 0.24 ms (before: each thread gathered its operand rows with
 // 2-byte loads), all nine layers of the network 81 -> 0.85 ms.
 //
+// At the volume's edges values of x that belong to no tap meet the zeros
+// outside it (u = 0 and g[-1], a tile's rows past ny), and zero times Inf or
+// NaN is NaN.  A CTA that drains a sum that is not finite sets *bad, and the
+// caller takes the gradient from the gather GEMM (k_conv.cu), whose products
+// are those of the pairs inside the volume.
+//
 // The CTAs share the tiles round robin, each sums all of its own in TMEM and
 // adds its sums to dw once.  Warp 0 loads, warp 1 issues the MMAs, all four
 // drain the sums.  Every wait is bounded; one that runs out sets *err, the
@@ -37,6 +43,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <cfloat>
 
 #include "net.h"
 #include "umma.cuh"
@@ -79,7 +86,7 @@ __device__ __forceinline__ uint64_t desc(uint32_t hi, uint32_t lo) {
 template <int MT, int KS>
 __global__ void __launch_bounds__(WG_THREADS, 1)
     k_wgrad_tma(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tg,
-                WgGeom g, float* __restrict__ dw, int* err) {
+                WgGeom g, float* __restrict__ dw, int* err, int* bad) {
   extern __shared__ uint8_t dsm[];
   __shared__ __align__(8) uint64_t full[WG_MAX_STAGES], empty[WG_MAX_STAGES], done;
   __shared__ uint32_t tslot;
@@ -196,6 +203,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
   umma::fence_after();
   if (!all_ok && threadIdx.x == 0) atomicExch(err, 1);
   if (all_ok && my_tiles > 0) {
+    float top = 0.0f;  // the largest |sum|; NaN stays
     for (int m = 0; m < MT; m++) {
       // row of D: core matrix r >> 3 = (dy * 3 + dz) * P + plane, channel r & 7
       const int r = m * 128 + warp * 32 + lane;
@@ -207,6 +215,9 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
         float v[16];
         umma::tmem_ld16(tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)(m * g.N + col), v);
         if (!own) continue;
+#pragma unroll
+        for (int e = 0; e < 16; e++)
+          asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(fabsf(v[e])));
 #pragma unroll
         for (int e = 0; e < 16; e++) {
           const int n = col + e;
@@ -231,6 +242,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
         }
       }
     }
+    if (!(top <= FLT_MAX)) *bad = 1;
   }
   umma::fence_before();
   __syncthreads();
@@ -290,7 +302,8 @@ cudaError_t conv3_pack_input(const bf16* src, int nx, int ny, int nz, int nb, bf
 }
 
 cudaError_t conv3_wgrad_tma(const bf16* x, int Cin, const bf16* gr, int Cout, int pack, int nx,
-                            int ny, int nz, int nb, float* dw, int* err, cudaStream_t st) {
+                            int ny, int nz, int nb, float* dw, int* err, int* bad,
+                            cudaStream_t st) {
   WgGeom g{};
   g.nz = nz;
   g.Cin = Cin;
@@ -358,7 +371,7 @@ cudaError_t conv3_wgrad_tma(const bf16* x, int Cin, const bf16* gr, int Cout, in
       !encode_planes(&mg, gr, planes_g, nx, ny, nz, nb, g.BX, g.Q, 1, 1))
     return cudaErrorInvalidValue;
   const size_t smem = WG_SMEM + 1024;
-  using Kern = void (*)(CUtensorMap, CUtensorMap, WgGeom, float*, int*);
+  using Kern = void (*)(CUtensorMap, CUtensorMap, WgGeom, float*, int*, int*);
   static constexpr Kern kerns[5][3] = {
       {k_wgrad_tma<1, 1>, k_wgrad_tma<1, 2>, k_wgrad_tma<1, 4>},
       {k_wgrad_tma<2, 1>, k_wgrad_tma<2, 2>, k_wgrad_tma<2, 4>},
@@ -376,7 +389,7 @@ cudaError_t conv3_wgrad_tma(const bf16* x, int Cin, const bf16* gr, int Cout, in
   const int gy = planes_x / g.P, gz = std::max(planes_g / g.Q, 1);
   const int ctas = std::max(1, std::min(g.ntiles, nsm / (gy * gz)));
   kern<<<dim3((unsigned)ctas, (unsigned)gy, (unsigned)gz), WG_THREADS, smem, st>>>(
-      mx, mg, g, dw, err);
+      mx, mg, g, dw, err, bad);
   return cudaGetLastError();
 }
 

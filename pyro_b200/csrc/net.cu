@@ -27,6 +27,9 @@ constexpr int MAX_VOLS = 64;
 // squared normalised residuals and their cell count, then per volume
 // (sum b^2, fluid cells)
 enum { SC_LOSS = 0, SC_GSQ = 1, SC_RES = 2, SC_RCNT = 3, SC_VOL = 4 };
+// and behind them an int per layer: its weight gradient has sums that are not
+// finite
+constexpr size_t SC_BYTES = (SC_VOL + 2 * MAX_VOLS) * 8 + NET_LAYERS * 4;
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -322,6 +325,19 @@ __global__ void __launch_bounds__(NT) k_bias_grad(const bf16* __restrict__ dz, s
   }
 }
 
+// Zeros over the weight gradients G of the layers (blockIdx.y) with bad[l] set.
+struct WOff {
+  int o[NET_LAYERS + 1];
+  explicit WOff(const size_t (&w)[NET_LAYERS + 1]) { std::copy(w, w + NET_LAYERS + 1, o); }
+};
+__global__ void __launch_bounds__(NT) k_clear_bad(WOff w, const int* __restrict__ bad,
+                                                  float* __restrict__ G) {
+  if (!bad[blockIdx.y]) return;
+  for (int i = w.o[blockIdx.y] + blockIdx.x * NT + threadIdx.x; i < w.o[blockIdx.y + 1];
+       i += gridDim.x * NT)
+    G[i] = 0.0f;
+}
+
 // phi = out * scale * s (fluid), 0 (solid); scale = out_scale * h^2
 // (160 x 320 x 160: 43 us with s per cell, 33 us with s per block)
 __global__ void __launch_bounds__(NT) k_output(const float* __restrict__ out,
@@ -491,7 +507,7 @@ int PyroNet::init() {
   if ((rc = master.alloc(n_params * 4)) || (rc = grad.alloc(n_params * 4)) ||
       (rc = adam_m.alloc(n_params * 4)) || (rc = adam_v.alloc(n_params * 4)) ||
       (rc = wbf.alloc(n_w * 2)) || (rc = wtf.alloc(n_w * 2)) || (rc = wtb.alloc(n_w * 2)) ||
-      (rc = scal.alloc((SC_VOL + 2 * MAX_VOLS) * 8)) ||
+      (rc = scal.alloc(SC_BYTES)) ||
       (rc = err.alloc(4)))
     return rc;
   if (cudaMallocHost(&host_scal, (SC_VOL + 2 * MAX_VOLS) * 8) != cudaSuccess) {
@@ -628,19 +644,20 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
       out.as<float>(), phi_t, flags, dv(v), S, (double)out_scale * h * h, (double)w_phi,
       (double)w_res, (double)out_scale, w_res > 0.0f ? res.as<float>() : nullptr, g9.as<bf16>());
   NET_CU(cudaGetLastError());
+  int* bad = reinterpret_cast<int*>(S + SC_VOL + 2 * MAX_VOLS);  // cleared by forward
+  struct Wg {
+    const bf16 *x, *g;
+    NetVol v;
+  } layers[NET_LAYERS];
   auto wg = [&](const DevBuf& x, const DevBuf& dz, int l, NetVol g) -> cudaError_t {
+    layers[l] = Wg{x.as<bf16>(), dz.as<bf16>(), g};
     const NetLayer& L = NET_SPEC[l];
     const bf16 *xs = x.as<bf16>(), *gs = dz.as<bf16>();
     cudaError_t e;
-    if (L.cout == 1)  // the last layer: pk holds its gradient's shifts
-      e = conv3_wgrad_tma(xs, L.cin, pk.as<bf16>(), 1, 1, g.nx, g.ny, g.nz, g.nb, G + w_off[l], E,
-                          st);
-    else if (L.cin == 2)  // the first: pk holds the input's
-      e = conv3_wgrad_tma(pk.as<bf16>(), 2, gs, L.cout, 2, g.nx, g.ny, g.nz, g.nb, G + w_off[l], E,
-                          st);
-    else
-      e = conv3_backward_weight(xs, L.cin, gs, L.cout, g.nx, g.ny, g.nz, g.nb, G + w_off[l], E,
-                                st);
+    // pk holds the shifts of the last layer's gradient, then the first's input
+    const int pack = L.cout == 1 ? 1 : L.cin == 2 ? 2 : 0;
+    e = conv3_wgrad_tma(pack == 2 ? pk.as<bf16>() : xs, L.cin, pack == 1 ? pk.as<bf16>() : gs,
+                        L.cout, pack, g.nx, g.ny, g.nz, g.nb, G + w_off[l], E, bad + l, st);
     if (e != cudaSuccess) return e;
     float* db = G + n_w + b_off[l];
     if (L.cout % 8 == 0)
@@ -685,7 +702,14 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
   NET_CU(bd(g2, 1, v, &e0a, g1));
   NET_CU(conv3_pack_input(in0.as<bf16>(), v.nx, v.ny, v.nz, v.nb, pk.as<bf16>(), st));
   NET_CU(wg(in0, g1, 0, v));
+  // layers with sums that are not finite, from the gather GEMM
+  k_clear_bad<<<dim3(8, NET_LAYERS), NT, 0, st>>>(WOff(w_off), bad, G);
   NET_CU(cudaGetLastError());
+  for (int l = 0; l < NET_LAYERS; l++) {
+    const Wg& a = layers[l];
+    NET_CU(conv3_wgrad_gather(a.x, NET_SPEC[l].cin, a.g, NET_SPEC[l].cout, a.v.nx, a.v.ny, a.v.nz,
+                              a.v.nb, G + w_off[l], E, bad + l, st));
+  }
   return PYRO_OK;
 }
 

@@ -43,9 +43,11 @@ cudaError_t conv3_backward_data(const __nv_bfloat16* dy, int Cout, int nx, int n
                                 int nb, const __nv_bfloat16* w, int Cin,
                                 const __nv_bfloat16* act, __nv_bfloat16* dx_bf16, float* dx_f32,
                                 int* err, cudaStream_t st);
-cudaError_t conv3_backward_weight(const __nv_bfloat16* x, int Cin, const __nv_bfloat16* dy,
-                                  int Cout, int nx, int ny, int nz, int nb, float* dw, int* err,
-                                  cudaStream_t st);
+// Weight gradient by the gather GEMM, accumulated into dw (FP32); nothing when
+// only_if is given and *only_if is 0.
+cudaError_t conv3_wgrad_gather(const __nv_bfloat16* x, int Cin, const __nv_bfloat16* dy, int Cout,
+                               int nx, int ny, int nz, int nb, float* dw, int* err,
+                               const int* only_if, cudaStream_t st);
 
 // Direct convolution on the CUDA cores for 2 -> 16 channels on [V][2] inputs
 // and 16 -> 1, FP32 sums in a fixed order.
@@ -75,11 +77,12 @@ void* tensor_map_encoder();
 // Weight gradient with TMA-staged operands (k_wgrad.cu), accumulated into dw
 // (FP32): input channels in planes of 8 and output channels a multiple of 16;
 // pack 1: one output channel, gr packed by conv3_pack_grad; pack 2: two input
-// channels, x packed by conv3_pack_input.
+// channels, x packed by conv3_pack_input.  *bad is set when a sum is not
+// finite: dw then holds NaN also where conv3_wgrad_gather does not.
 bool conv3_wgrad_fits(int Cin, int Cout);
 cudaError_t conv3_wgrad_tma(const __nv_bfloat16* x, int Cin, const __nv_bfloat16* gr, int Cout,
                             int pack, int nx, int ny, int nz, int nb, float* dw, int* err,
-                            cudaStream_t st);
+                            int* bad, cudaStream_t st);
 // The three x-shifts of a gradient of one channel ([V]) or of an input of two
 // ([V][2]) as one plane of 8 channels, 0 outside the row and past the shifts:
 // dst[u][j] = src[u - (j - 1)], dst[u][2 j + c] = src[u + j - 1][c].

@@ -285,3 +285,40 @@ def test_backward_data_not_finite_stays_local(lib, Cin, Cout, dims):
     for o in out[1:]:
         assert not torch.isfinite(o[near][on[near]]).any()
         assert (o[near][~on[near]] == 0).all()
+
+
+@pytest.mark.parametrize("Cin,Cout,dims", [(16, 16, (5, 9, 33)),    # ragged tiles in x and y
+                                           (8, 32, (4, 18, 20)),
+                                           (16, 80, (4, 6, 20)),    # a width that the gather pads
+                                           (48, 16, (24, 30, 64))])  # several tiles per CTA
+@pytest.mark.parametrize("which", ["x", "dy"])
+def test_backward_weight_not_finite_stays_local(lib, Cin, Cout, dims, which):
+    """Voxels on the volume's edges that are not finite: an x reaches the entries
+    that a pair of voxels inside the volume has it in, and no other; a dy the
+    entries of its channel (with the zeros around x in all taps).  The others
+    are the sums of the finite tensors (FP32 sums in another order, as above)."""
+    nz, ny, nx = dims
+    t = {"x": _tensors(1, Cin, nz, ny, nx, 1, 41)[0], "dy": _tensors(1, Cout, nz, ny, nx, 1, 42)[0]}
+    at = [(nz - 1, ny - 1, nx - 1), (0, ny // 2, 0), (nz // 2, 0, nx - 1)]
+    w = torch.zeros(Cout, Cin, 3, 3, 3, device="cuda", requires_grad=True)
+    Fn.conv3d(t["x"], w, None, padding=1).backward(t["dy"])
+    ref = w.grad.permute(0, 2, 3, 4, 1).reshape(Cout, 27, Cin)
+    hit = torch.zeros(Cout, 27, Cin, dtype=torch.bool, device="cuda")
+    bad = t[which].clone()
+    for k, ((z, y, x), v) in enumerate(zip(at, (float("nan"), float("inf"), -float("inf")))):
+        c = 3 + 2 * k
+        bad[0, c, z, y, x] = v
+        for tap in range(27):  # x at v meets dy at v - tap
+            d = (tap // 9 - 1, tap // 3 % 3 - 1, tap % 3 - 1)
+            if which == "dy":
+                hit[c, tap] = True
+            elif all(0 <= p - s < n for p, s, n in zip((z, y, x), d, dims)):
+                hit[:, tap, c] = True
+    t[which] = bad
+    xc, dc = _cl(t["x"]), _cl(t["dy"])
+    dw = torch.zeros(Cout, 27, Cin, device="cuda")
+    rc = lib.pyro_conv3_backward_weight(ptr(xc), Cin, ptr(dc), Cout, nx, ny, nz, 1, ptr(dw), None)
+    assert rc == 0, lib.pyro_last_error()
+    assert not torch.isfinite(dw[hit]).any()
+    assert torch.isfinite(dw[~hit]).all()
+    _close(dw[~hit], ref[~hit])
