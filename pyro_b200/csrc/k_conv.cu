@@ -425,11 +425,11 @@ __global__ void k_wprep(const bf16* __restrict__ w, int Cout, int Cin, int backw
 }
 
 // dw += s, nothing when *bad is set
-__global__ void __launch_bounds__(256) k_add_unless(const float* __restrict__ s, int n,
+__global__ void __launch_bounds__(256) k_add_unless(const double* __restrict__ s, int n,
                                                     const int* __restrict__ bad,
                                                     float* __restrict__ dw) {
   const int i = blockIdx.x * 256 + threadIdx.x;
-  if (i < n && !*bad) dw[i] += s[i];
+  if (i < n && !*bad) dw[i] = (float)((double)dw[i] + s[i]);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -480,6 +480,13 @@ cudaError_t conv3_backward_data(const bf16* dy, int Cout, int nx, int ny, int nz
   return gemm_dispatch(npad, grid, ld, ep, ksteps, ksteps, err, st);
 }
 
+int conv3_gather_steps(int Cin, long V) {
+  const long ksteps = (V + 15) / 16, mt = (27 * Cin + 127) / 128;
+  // split K so that the grid covers the GPU a few times over
+  const long splits = std::max(1l, std::min(ksteps, (148 * 8) / std::max(mt, 1l)));
+  return (int)((ksteps + splits - 1) / splits);
+}
+
 // dw[co][tap][ci] += sum_voxels dy[v][co] x[v + tap][ci]  (dw FP32).
 cudaError_t conv3_wgrad_gather(const bf16* x, int Cin, const bf16* dy, int Cout, int nx, int ny,
                                int nz, int nb, float* dw, int* err, const int* only_if,
@@ -489,12 +496,8 @@ cudaError_t conv3_wgrad_gather(const bf16* x, int Cin, const bf16* dy, int Cout,
   int M = 27 * Cin;
   int npad = pad16(Cout);
   if (only_if && npad > 64) npad = npad > 96 ? 128 : 96;  // behind the boxes, which take 80 and 112
-  int ksteps = (V + 15) / 16;
-  int mt = (M + 127) / 128;
-  // split K so that the grid covers the GPU a few times over
-  int splits = std::max(1, std::min(ksteps, (148 * 8) / std::max(mt, 1)));
-  int kpc = (ksteps + splits - 1) / splits;
-  splits = (ksteps + kpc - 1) / kpc;
+  const int ksteps = (V + 15) / 16, mt = (M + 127) / 128, kpc = conv3_gather_steps(Cin, V);
+  const int splits = (ksteps + kpc - 1) / kpc;
   WgradLoad ld{x, dy, g, Cin, Cout, npad};
   WgradEpi ep{dw, M, Cout};
   dim3 grid(mt, splits, 1);
@@ -630,13 +633,13 @@ int pyro_conv3_backward_weight(const void* x, int Cin, const void* dy, int Cout,
   const bool boxes = conv3_wgrad_fits(Cin, Cout) && at % 16 == 0;
   const int n = Cout * 27 * Cin;
   DevBuf err;  // the error and bad flags, then the boxes' sums
-  int rc = err.alloc(16 + (boxes ? (size_t)n * 4 : 0));
+  int rc = err.alloc(16 + (boxes ? (size_t)n * 8 : 0));
   if (rc != PYRO_OK) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   int *E = err.as<int>(), *bad = boxes ? E + 1 : nullptr;
   cudaError_t e = cudaSuccess;
   if (boxes) {
-    float* sums = err.as<float>() + 4;
+    double* sums = err.as<double>() + 2;
     e = conv3_wgrad_tma((const bf16*)x, Cin, (const bf16*)dy, Cout, 0, nx, ny, nz, nb, sums, E,
                         bad, st);
     if (e == cudaSuccess) {

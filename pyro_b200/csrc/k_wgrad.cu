@@ -26,7 +26,7 @@
 // channels need 5.8 cycles per voxel and SM; the kernel issues one every 54.
 // Measured on two 128^3 volumes: 16 -> 16 channels 16.4 ms -> 0.12 ms, 48 ->
 // 16 47 ms -> 0.24 ms (before: each thread gathered its operand rows with
-// 2-byte loads), all nine layers of the network 81 -> 0.85 ms.
+// 2-byte loads), all nine layers of the network 81 -> 0.92 ms.
 //
 // At the volume's edges values of x that belong to no tap meet the zeros
 // outside it (u = 0 and g[-1], a tile's rows past ny), and zero times Inf or
@@ -34,8 +34,13 @@
 // caller takes the gradient from the gather GEMM (k_conv.cu), whose products
 // are those of the pairs inside the volume.
 //
-// The CTAs share the tiles round robin, each sums all of its own in TMEM and
-// adds its sums to dw once.  Warp 0 loads, warp 1 issues the MMAs, all four
+// The CTAs share the tiles round robin; each takes its own in turn into as many
+// accumulators as the TMEM holds, and adds their sums to dw, in FP64, once.  A
+// sum's error grows with the MMAs that add to it (1.8e-8 of it for each on
+// normal inputs: 16 -> 16 channels on two 128^3 volumes 3.2e-5 with one
+// accumulator of 1,771, 6.1e-6 with five), so no accumulator takes more of them
+// than one of the gather GEMM's (k_conv.cu), whose error that bounds: past it
+// there are more CTAs than SMs.  Warp 0 loads, warp 1 issues the MMAs, all four
 // drain the sums.  Every wait is bounded; one that runs out sets *err, the
 // copies in flight land (bounded again) and the TMEM is freed.
 #include <cuda.h>
@@ -65,6 +70,7 @@ struct WgGeom {
   int Cin, Cout;        // of dw
   int pack;             // 0; 1: g's channel is the x-shift; 2: x's channels are (x-shift, ci)
   int stages;
+  int nacc;             // accumulators, taken in turn
   uint32_t xbytes, stage_bytes, ncols;
 };
 
@@ -82,11 +88,11 @@ __device__ __forceinline__ uint64_t desc(uint32_t hi, uint32_t lo) {
 // MT: M tiles; KS: K steps of 16 voxels in a row.  Both are compile-time so
 // that a row's MMAs are one unrolled run: with loops around single MMAs the
 // issuing thread took 170 cycles for each (322 us for 16 -> 16 channels on
-// two 128^3 volumes, @16@ us unrolled).
+// two 128^3 volumes, 115 us unrolled).
 template <int MT, int KS>
 __global__ void __launch_bounds__(WG_THREADS, 1)
     k_wgrad_tma(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUtensorMap tg,
-                WgGeom g, float* __restrict__ dw, int* err, int* bad) {
+                WgGeom g, double* __restrict__ dw, int* err, int* bad) {
   extern __shared__ uint8_t dsm[];
   __shared__ __align__(8) uint64_t full[WG_MAX_STAGES], empty[WG_MAX_STAGES], done;
   __shared__ uint32_t tslot;
@@ -166,8 +172,9 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     const uint32_t grow = (uint32_t)(g.ndx * g.Q) * row >> 4;  // g rows per y
     constexpr uint32_t MSTEP = 16u * KS * 16u;                 // 16 rows of x
     const uint32_t ncol = (uint32_t)g.N;
-    uint32_t acc = 0u, phase = 0u;
-    int s = 0;
+    const uint32_t sums = (uint32_t)(MT * g.N);  // columns of an accumulator
+    uint32_t phase = 0u;
+    int s = 0, a = 0;
     for (int i = 0; i < my_tiles; i++) {
       if (abort_flag) break;
       if (!umma::mbar_wait_warp(&full[s], phase)) {
@@ -177,6 +184,8 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
       umma::fence_after();
       const uint32_t sx = umma::smem_u32(base) + (uint32_t)s * g.stage_bytes;
       uint32_t ax = desc_lo(sx), bg = desc_lo(sx + g.xbytes);
+      uint32_t acc = i < g.nacc ? 0u : 1u;
+      const uint32_t dt = tbase + (uint32_t)a * sums;
 #pragma unroll 1
       for (int y = 0; y < g.BY; y++) {
         if (umma::elect_one()) {
@@ -184,7 +193,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
           for (int k = 0; k < KS; k++)
 #pragma unroll
             for (int m = 0; m < MT; m++)
-              umma::mma_bf16(tbase + m * ncol, desc(hi, ax + k * 16u + m * MSTEP),
+              umma::mma_bf16(dt + m * ncol, desc(hi, ax + k * 16u + m * MSTEP),
                              desc(hi, bg + k * 16u), idesc, k ? 1u : acc);
         }
         acc = 1u;
@@ -193,6 +202,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
       }
       if (umma::elect_one()) umma::mma_commit(&empty[s]);
       if (++s == S) s = 0, phase ^= 1u;
+      if (++a == g.nacc) a = 0;
     }
     if (!ok) abort_flag = 1;
     // every MMA issued has finished before the sums are read
@@ -212,8 +222,15 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
       const int dy = q / 3, dz = q - 3 * dy;
       const int c8 = (p0 + pl) * 8 + (r & 7);
       for (int col = 0; col < g.N; col += 16) {
+        const uint32_t tv = tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)(m * g.N + col);
         float v[16];
-        umma::tmem_ld16(tbase + ((uint32_t)(warp * 32) << 16) + (uint32_t)(m * g.N + col), v);
+        umma::tmem_ld16(tv, v);
+        for (int a = 1; a < min(g.nacc, my_tiles); a++) {
+          float t[16];
+          umma::tmem_ld16(tv + (uint32_t)(a * MT * g.N), t);
+#pragma unroll
+          for (int e = 0; e < 16; e++) v[e] += t[e];
+        }
         if (!own) continue;
 #pragma unroll
         for (int e = 0; e < 16; e++)
@@ -238,7 +255,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
             ci = c8;
           }
           if (co < g.Cout && ci < g.Cin)
-            atomicAdd(dw + ((size_t)co * 27 + (dz * 3 + dy) * 3 + dx) * g.Cin + ci, v[e]);
+            atomicAdd(dw + ((size_t)co * 27 + (dz * 3 + dy) * 3 + dx) * g.Cin + ci, (double)v[e]);
         }
       }
     }
@@ -302,7 +319,7 @@ cudaError_t conv3_pack_input(const bf16* src, int nx, int ny, int nz, int nb, bf
 }
 
 cudaError_t conv3_wgrad_tma(const bf16* x, int Cin, const bf16* gr, int Cout, int pack, int nx,
-                            int ny, int nz, int nb, float* dw, int* err, int* bad,
+                            int ny, int nz, int nb, double* dw, int* err, int* bad,
                             cudaStream_t st) {
   WgGeom g{};
   g.nz = nz;
@@ -321,6 +338,10 @@ cudaError_t conv3_wgrad_tma(const bf16* x, int Cin, const bf16* gr, int Cout, in
   // loads (BY + 2) / BY of x, and a box of g costs the same for any width:
   // 16 -> 16 channels 107 us against 140 with 32), else the tallest tile of
   // the widest (48 -> 16: 243 us with 32 x 4, 294 with 64 x 1).
+  // MMAs that an accumulator takes at most: the gather GEMM's, or 8, whose error
+  // is below that of its additions of more CTAs' sums in FP32
+  const long V = (long)nx * ny * nz * nb;
+  const int most = std::max(conv3_gather_steps(Cin, V), 8);
   bool found = false;
   for (int P = std::min(planes_x, 8); P >= 1 && !found; P--) {
     if (planes_x % P) continue;
@@ -335,7 +356,7 @@ cudaError_t conv3_wgrad_tma(const bf16* x, int Cin, const bf16* gr, int Cout, in
         // x: into the stage's g and the slack after the last stage
         const uint32_t slack = (uint32_t)(16 * mt - 9 * P) * row;
         for (int BY : {8, 4, 2, 1}) {
-          if (BY > 1 && BY / 2 >= ny) continue;
+          if (BY > 1 && (BY / 2 >= ny || BY * (BX / 16) > most)) continue;
           const uint32_t xb = (uint32_t)((BY + 2) * 3 * P) * row;
           const uint32_t sb = xb + (uint32_t)(BY * g.ndx * g.Q) * row;
           if (slack >= WG_SMEM || (WG_SMEM - slack) / sb < (uint32_t)want) continue;
@@ -359,8 +380,9 @@ cudaError_t conv3_wgrad_tma(const bf16* x, int Cin, const bf16* gr, int Cout, in
     }
   }
   if (!found) return cudaErrorInvalidValue;
+  g.nacc = std::min(512 / (g.mt * g.N), 16);
   g.ncols = 32;
-  while ((int)g.ncols < g.mt * g.N) g.ncols *= 2;
+  while ((int)g.ncols < g.nacc * g.mt * g.N) g.ncols *= 2;
   g.tiles_x = (nx + g.BX - 1) / g.BX;
   g.tiles_y = (ny + g.BY - 1) / g.BY;
   const long nt = (long)g.tiles_x * g.tiles_y * nz * nb;
@@ -371,7 +393,7 @@ cudaError_t conv3_wgrad_tma(const bf16* x, int Cin, const bf16* gr, int Cout, in
       !encode_planes(&mg, gr, planes_g, nx, ny, nz, nb, g.BX, g.Q, 1, 1))
     return cudaErrorInvalidValue;
   const size_t smem = WG_SMEM + 1024;
-  using Kern = void (*)(CUtensorMap, CUtensorMap, WgGeom, float*, int*, int*);
+  using Kern = void (*)(CUtensorMap, CUtensorMap, WgGeom, double*, int*, int*);
   static constexpr Kern kerns[5][3] = {
       {k_wgrad_tma<1, 1>, k_wgrad_tma<1, 2>, k_wgrad_tma<1, 4>},
       {k_wgrad_tma<2, 1>, k_wgrad_tma<2, 2>, k_wgrad_tma<2, 4>},
@@ -387,7 +409,8 @@ cudaError_t conv3_wgrad_tma(const bf16* x, int Cin, const bf16* gr, int Cout, in
   if (cudaGetDevice(&dev) == cudaSuccess)
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const int gy = planes_x / g.P, gz = std::max(planes_g / g.Q, 1);
-  const int ctas = std::max(1, std::min(g.ntiles, nsm / (gy * gz)));
+  const int per = g.nacc * std::max(1, most / (g.BY * (g.BX / 16)));  // tiles of a CTA at most
+  const int ctas = std::max({1, std::min(g.ntiles, nsm / (gy * gz)), (g.ntiles + per - 1) / per});
   kern<<<dim3((unsigned)ctas, (unsigned)gy, (unsigned)gz), WG_THREADS, smem, st>>>(
       mx, mg, g, dw, err, bad);
   return cudaGetLastError();

@@ -325,17 +325,19 @@ __global__ void __launch_bounds__(NT) k_bias_grad(const bf16* __restrict__ dz, s
   }
 }
 
-// Zeros over the weight gradients G of the layers (blockIdx.y) with bad[l] set.
+// The weight gradients G of the layers (blockIdx.y) from their sums; zeros where
+// bad[l] is set.
 struct WOff {
   int o[NET_LAYERS + 1];
   explicit WOff(const size_t (&w)[NET_LAYERS + 1]) { std::copy(w, w + NET_LAYERS + 1, o); }
 };
-__global__ void __launch_bounds__(NT) k_clear_bad(WOff w, const int* __restrict__ bad,
+__global__ void __launch_bounds__(NT) k_wgrad_out(WOff w, const double* __restrict__ sums,
+                                                  const int* __restrict__ bad,
                                                   float* __restrict__ G) {
-  if (!bad[blockIdx.y]) return;
+  const bool no = bad[blockIdx.y] != 0;
   for (int i = w.o[blockIdx.y] + blockIdx.x * NT + threadIdx.x; i < w.o[blockIdx.y + 1];
        i += gridDim.x * NT)
-    G[i] = 0.0f;
+    G[i] = no ? 0.0f : (float)sums[i];
 }
 
 // phi = out * scale * s (fluid), 0 (solid); scale = out_scale * h^2
@@ -555,10 +557,11 @@ int PyroNet::ensure(NetVol v, bool bwd) {
   if (bwd) {
     for (auto& a : bw)
       if ((rc = a.b->alloc(a.n * 2))) return rc;
-    if ((rc = res.alloc(V0 * 4))) return rc;
+    if ((rc = res.alloc(V0 * 4)) || (rc = wsum.alloc(n_w * 8))) return rc;
   } else {
     for (auto& a : bw) a.b->release();
     res.release();
+    wsum.release();
   }
   vol = v;
   has_bwd = bwd;
@@ -637,6 +640,7 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
   int* E = err.as<int>();
   float* G = grad.as<float>();
   NET_CU(cudaMemsetAsync(grad.p, 0, grad.bytes, st));
+  NET_CU(cudaMemsetAsync(wsum.p, 0, wsum.bytes, st));
   if (w_res > 0.0f)
     k_res<<<blocks_for(cells * v.nb), NT, 0, st>>>(out.as<float>(), b, flags, dv(v), S,
                                                    (double)out_scale, res.as<float>());
@@ -657,7 +661,8 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
     // pk holds the shifts of the last layer's gradient, then the first's input
     const int pack = L.cout == 1 ? 1 : L.cin == 2 ? 2 : 0;
     e = conv3_wgrad_tma(pack == 2 ? pk.as<bf16>() : xs, L.cin, pack == 1 ? pk.as<bf16>() : gs,
-                        L.cout, pack, g.nx, g.ny, g.nz, g.nb, G + w_off[l], E, bad + l, st);
+                        L.cout, pack, g.nx, g.ny, g.nz, g.nb, wsum.as<double>() + w_off[l], E, bad + l,
+                        st);
     if (e != cudaSuccess) return e;
     float* db = G + n_w + b_off[l];
     if (L.cout % 8 == 0)
@@ -702,9 +707,9 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
   NET_CU(bd(g2, 1, v, &e0a, g1));
   NET_CU(conv3_pack_input(in0.as<bf16>(), v.nx, v.ny, v.nz, v.nb, pk.as<bf16>(), st));
   NET_CU(wg(in0, g1, 0, v));
-  // layers with sums that are not finite, from the gather GEMM
-  k_clear_bad<<<dim3(8, NET_LAYERS), NT, 0, st>>>(WOff(w_off), bad, G);
+  k_wgrad_out<<<dim3(64, NET_LAYERS), NT, 0, st>>>(WOff(w_off), wsum.as<double>(), bad, G);
   NET_CU(cudaGetLastError());
+  // layers with sums that are not finite, from the gather GEMM
   for (int l = 0; l < NET_LAYERS; l++) {
     const Wg& a = layers[l];
     NET_CU(conv3_wgrad_gather(a.x, NET_SPEC[l].cin, a.g, NET_SPEC[l].cout, a.v.nx, a.v.ny, a.v.nz,

@@ -56,6 +56,9 @@ cudaError_t conv3_direct(const __nv_bfloat16* x, int C, int nx, int ny, int nz, 
                          const __nv_bfloat16* w, int Cout, const float* bias, int relu,
                          __nv_bfloat16* y_bf16, float* y_f32, cudaStream_t st);
 
+// K steps of 16 voxels that one of its sums takes, for V voxels.
+int conv3_gather_steps(int Cin, long V);
+
 // TMA-staged convolution (k_conv3.cu) on tap-major weights prepared by
 // conv3_prep_weights: input channels K a multiple of 16, or (pack) the one
 // channel of a tensor packed by conv3_pack_grad.  fine (BF16
@@ -75,13 +78,13 @@ cudaError_t conv3_tma(const __nv_bfloat16* x, int K, bool pack, int nx, int ny, 
 void* tensor_map_encoder();
 
 // Weight gradient with TMA-staged operands (k_wgrad.cu), accumulated into dw
-// (FP32): input channels in planes of 8 and output channels a multiple of 16;
+// (FP64): input channels in planes of 8 and output channels a multiple of 16;
 // pack 1: one output channel, gr packed by conv3_pack_grad; pack 2: two input
 // channels, x packed by conv3_pack_input.  *bad is set when a sum is not
 // finite: dw then holds NaN also where conv3_wgrad_gather does not.
 bool conv3_wgrad_fits(int Cin, int Cout);
 cudaError_t conv3_wgrad_tma(const __nv_bfloat16* x, int Cin, const __nv_bfloat16* gr, int Cout,
-                            int pack, int nx, int ny, int nz, int nb, float* dw, int* err,
+                            int pack, int nx, int ny, int nz, int nb, double* dw, int* err,
                             int* bad, cudaStream_t st);
 // The three x-shifts of a gradient of one channel ([V]) or of an input of two
 // ([V][2]) as one plane of 8 channels, 0 outside the row and past the shifts:
@@ -126,6 +129,7 @@ struct PyroNet {
   __nv_bfloat16* skip1() const {
     return c1.as<__nv_bfloat16>() + (size_t)8 * vol.half().voxels() * 8;
   }
+  pyro::DevBuf wsum;  // weight gradients' sums in FP64 (backward)
   pyro::DevBuf pk;  // packed x-shifts of the output gradient, then of the input (backward)
   pyro::DevBuf g9, g8, gc0, g7, gc1, g6, g5, gp2, g4, g3, gp1, g2, g1;
   cudaStream_t stream = nullptr;

@@ -322,3 +322,30 @@ def test_backward_weight_not_finite_stays_local(lib, Cin, Cout, dims, which):
     assert not torch.isfinite(dw[hit]).any()
     assert torch.isfinite(dw[~hit]).all()
     _close(dw[~hit], ref[~hit])
+
+
+@pytest.mark.parametrize("Cin,Cout,dims", [(16, 16, (64, 64, 128)), (48, 16, (40, 64, 64)),
+                                           (16, 32, (30, 37, 130))])
+def test_backward_weight_error_bounded_by_the_gather(lib, Cin, Cout, dims):
+    """Sums over many voxels: the TMA-staged gradient is no further from 64 bits
+    than the gather GEMM's, which the same values off a 16-byte boundary take."""
+    nz, ny, nx = dims
+    g = torch.Generator(device="cuda").manual_seed(51)
+    x = torch.randn(1, Cin, nz, ny, nx, device="cuda", generator=g).abs().bfloat16().float()
+    dy = torch.randn(1, Cout, nz, ny, nx, device="cuda", generator=g).bfloat16().float()
+    ref = torch.empty(Cout, 27, Cin, dtype=torch.float64, device="cuda")
+    xp, d = Fn.pad(x, (1,) * 6).double()[0], dy.double().reshape(Cout, -1)
+    for t in range(27):
+        z0, y0, x0 = t // 9, t // 3 % 3, t % 3
+        ref[:, t] = d @ xp[:, z0:z0 + nz, y0:y0 + ny, x0:x0 + nx].reshape(Cin, -1).t()
+    xc, dc = _cl(x).reshape(-1), _cl(dy)
+    off = torch.zeros(xc.numel() + 8, dtype=xc.dtype, device="cuda")[1:]
+    off[:xc.numel()] = xc
+    errs = []
+    for xv in (xc, off):
+        dw = torch.zeros(Cout, 27, Cin, device="cuda")
+        rc = lib.pyro_conv3_backward_weight(ptr(xv), Cin, ptr(dc), Cout, nx, ny, nz, 1, ptr(dw),
+                                            None)
+        assert rc == 0, lib.pyro_last_error()
+        errs.append(((dw - ref).norm() / ref.norm()).item())
+    assert errs[0] <= errs[1], errs
