@@ -110,9 +110,10 @@ __global__ void __launch_bounds__(256) k_mg_resid(Lvl d, float h2, const float* 
 // ------------------------------------------------------------ coarse solve
 // The coarsest level is swept 80 times per V-cycle (src/sim.rs:473), 160
 // dependent red-black passes over ~1-30 k cells.  One thread-block cluster
-// runs them all in a single launch: CTA r owns z-planes [r nz / C,
-// (r + 1) nz / C) of phi in its shared memory, with a ghost plane on either
-// side.
+// runs them all in a single launch: CTA r of the C that own planes (one plane
+// each at least; a cluster's further CTAs only join its barriers) owns z-planes
+// [r nz / C, (r + 1) nz / C) of phi in its shared memory, with a ghost plane on
+// either side.
 //
 // What bounds it is the latency of a pass, so a pass costs one block barrier
 // and one message to each neighbour: a thread that has updated a cell of the
@@ -228,8 +229,13 @@ __global__ void __launch_bounds__(coarse_threads(K), 1)
   __shared__ __align__(8) uint64_t bar[2];
   __shared__ float zero;
   const int T = (int)blockDim.x;
-  const int C = (int)cl.num_blocks();
+  const int C = min((int)cl.num_blocks(), d.nz);
   const int rank = (int)cl.block_rank();
+  if (rank >= C) {  // no planes
+    cl.sync();
+    cl.sync();
+    return;
+  }
   const int z0 = rank * d.nz / C, z1 = (rank + 1) * d.nz / C, planes = z1 - z0;
   const int hxn = (d.nx + 1) / 2, pl = hxn * d.ny;
   const int cap = ((d.nz + C - 1) / C + 2) * pl;  // floats of one colour, the same in every CTA
@@ -394,34 +400,35 @@ __global__ void k_bf16_to_f32(const __nv_bfloat16* __restrict__ a, float* __rest
 
 // Shared memory of a CTA: two colours of its planes and two ghost planes.
 size_t coarse_smem(Dims3 d, int C) {
+  C = std::min(C, d.nz);
   return (size_t)((d.nz + C - 1) / C + 2) * ((d.nx + 1) / 2) * d.ny * 2 * 4;
 }
 
 // Cluster size, cells per thread and colour and threads per CTA for a level;
-// C = 0 when none fits.  The largest cluster: a message to a neighbour costs
-// less than the warps that more planes per CTA would add (20 x 30 x 20: 67 us
-// on 16 CTAs, 89 on 8; 8 x 20 x 8: 43 us on 8, 44 on 4).  As few
-// cells per thread as fit: the same cells in fewer warps wait longer (two per
-// thread instead of one: 20 x 40 x 20 88 us against 82, 16 x 30 x 16 65
+// C = 0 when it does not fit.  A CTA per plane, up to the largest cluster: a
+// message to a neighbour costs less than the warps that more planes per CTA
+// would add (20 x 30 x 20: 67 us on 16 CTAs, 89 on 8; 20 x 40 x 12: 63 us on
+// 16 of which 12 have a plane, 84 on 8; 16 x 32 x 6: 51 us on 8, 62 on 4).  As
+// few cells per thread as fit: the same cells in fewer warps wait longer (two
+// per thread instead of one: 20 x 40 x 20 88 us against 82, 16 x 30 x 16 65
 // against 53).
 struct CoarsePlan {
   int C = 0, K = 0, T = 0;
 };
 CoarsePlan coarse_plan(Dims3 d, int max_cluster) {
   CoarsePlan pl;
-  for (int C : {COARSE_MAX_CLUSTER, 8, 4, 2}) {
-    if (C > max_cluster || C > d.nz) continue;
-    const int planes = (d.nz + C - 1) / C;
-    const int vpc = (d.nx + 1) / 2 * d.ny * planes;
-    if (coarse_smem(d, C) > (size_t)COARSE_SMEM) continue;
-    for (int K : {1, 2, 4}) {
-      const int T = ((vpc + K - 1) / K + 31) / 32 * 32;
-      if (T > coarse_threads(K)) continue;
-      pl.C = C;
-      pl.K = K;
-      pl.T = T;
-      return pl;
-    }
+  int C = 2;
+  while (C < max_cluster && C < d.nz) C *= 2;
+  const int planes = (d.nz + C - 1) / C;
+  const long vpc = (long)((d.nx + 1) / 2) * d.ny * planes;
+  if (coarse_smem(d, C) > (size_t)COARSE_SMEM) return pl;
+  for (int K : {1, 2, 4}) {
+    const long T = ((vpc + K - 1) / K + 31) / 32 * 32;
+    if (T > coarse_threads(K)) continue;
+    pl.C = C;
+    pl.K = K;
+    pl.T = (int)T;
+    return pl;
   }
   return pl;
 }

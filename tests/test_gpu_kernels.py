@@ -451,6 +451,36 @@ def test_mg_coarse_solve_cluster_shapes(lib, nx, ny, nz, seed, h):
     assert np.array_equal(host(pd), e)
 
 
+@pytest.mark.parametrize("nx,ny,nz", [
+    (48, 48, 12), (40, 52, 14), (44, 48, 9),  # fewer planes than a cluster has CTAs,
+    (64, 40, 12), (40, 80, 9), (60, 60, 6),   # 1,025 to 2,048 cells of a colour in each
+    (60, 60, 3), (60, 64, 2)])
+@pytest.mark.parametrize("bc_mode", [0, 1])
+def test_mg_coarse_solve_of_few_large_planes(lib, nx, ny, nz, bc_mode):
+    """Levels of a plane per CTA, in clusters with CTAs that have none: the
+    coarse solve's two orders bit for bit one pass launch per colour."""
+    h, om, its = 0.16, 1.6, 6
+    rng = np.random.default_rng(nx * ny + nz)
+    f = dev((rng.random((nz, ny, nx)) < 0.15).astype(np.uint32))
+    b = dev(rng.normal(0, 1, (nz, ny, nx)).astype(np.float32))
+    p = rng.normal(0, 0.1, (nz, ny, nx)).astype(np.float32)
+    meta = dev(np.zeros((nz, ny, nx), np.uint8))
+    assert lib.pyro_k_mg_meta(nx, ny, nz, ptr(f), ptr(meta), None) == 0
+    for sym in (False, True) if bc_mode == 0 else (True,):
+        got, want = dev(p), dev(p)
+        if sym:
+            rc = lib.pyro_k_mg_coarse_sym(nx, ny, nz, h, ptr(b), ptr(f), ptr(got), its, om,
+                                          bc_mode, None)
+        else:
+            rc = lib.pyro_k_mg_coarse(nx, ny, nz, h, ptr(b), ptr(f), ptr(got), its, om, None)
+        assert rc == 0, lib.pyro_last_error()
+        for it in range(its):
+            for c in ((1, 0) if sym and it & 1 else (0, 1)):
+                assert lib.pyro_k_mg_pass(nx, ny, nz, h, ptr(b), ptr(meta), ptr(want), c, om,
+                                          bc_mode, _abi.MG_F32, None) == 0
+        assert np.array_equal(host(got), host(want))
+
+
 @pytest.mark.parametrize("nx,ny,nz,seed,h", [(20, 40, 20, 8, 0.16), (32, 32, 22, 9, 0.2),
                                              (8, 20, 8, 10, 0.32)])
 @pytest.mark.parametrize("bc_mode", [0, 1])
