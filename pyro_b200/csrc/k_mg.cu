@@ -519,14 +519,23 @@ cudaError_t mg_sweeps_t(Dims3 d, float h, const TS* b, const uint8_t* meta, TS* 
 
 bool mg_coarse_fits(Dims3 d) { return coarse_cluster_size(d) != 0; }
 
-// Levels with one cell of a colour per thread: a launch sets its cells up once
-// for all passes (16 to 32 k cells: MGPCG on 256^3 13.50 -> 13.30 ms, on 75 x
-// 183 x 75 a 4 cm frame 4.96 -> 4.86 ms), but four cells per thread make a pass
-// longer than a launch (32 x 60 x 32 in the V-cycles on 128 x 240 x 128: 1043
-// us against 968 with a launch per pass).
+// Levels with one cell of a colour per thread: four cells per thread make a
+// pass longer than a launch (32 x 60 x 32 in the V-cycles on 128 x 240 x 128:
+// 1043 us against 968 with a launch per pass).
 bool mg_sweeps_fit(Dims3 d) {
   const CoarsePlan pl = coarse_plan(d, coarse_max_cluster());
   return pl.C != 0 && pl.K == 1;
+}
+
+// A launch sets its cells up once for all passes, which pays for the eight of
+// MGPCG's smoother on every level that fits (us, cluster against passes: 16 x 40
+// x 16 7.7 / 12.6, 19 x 46 x 19 11.1 / 12.1, 40 x 50 x 16 12.2 / 13.7, BF16 11.1
+// / 14.0 and 12.4 / 12.5) and for the four of the V-cycles up to 320 cells of a
+// colour per CTA (16 x 32 x 16 6.2 / 6.3, 16 x 40 x 16 6.4 / 6.4; beyond, 16 x
+// 48 x 16 6.7 / 6.3, 19 x 46 x 19 9.0 / 5.8).
+bool mg_sweeps_pay(Dims3 d, int passes) {
+  const CoarsePlan pl = coarse_plan(d, coarse_max_cluster());
+  return pl.C != 0 && pl.K == 1 && (passes >= 8 || pl.T <= 320);
 }
 
 cudaError_t launch_mg_sweeps(Dims3 d, float h, const void* b, const uint8_t* meta, void* p,

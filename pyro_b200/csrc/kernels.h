@@ -121,6 +121,7 @@ cudaError_t launch_mg_resid(Dims3 d, float h, const float* p, const float* b, co
 // that fits a thread-block cluster, in one launch; equal to launch_mg_pass /
 // launch_mg_pass_bf16 once per colour, bit for bit.
 bool mg_sweeps_fit(Dims3 d);
+bool mg_sweeps_pay(Dims3 d, int passes);  // fits, and is faster than a launch per pass
 cudaError_t launch_mg_sweeps(Dims3 d, float h, const void* b, const uint8_t* meta, void* p,
                              int iters, float omega, int black_first, int bc_mode, bool bf16,
                              cudaStream_t st);

@@ -134,8 +134,6 @@ int Multigrid::init(Dims3 d0, float h0, int bc, size_t direct_max) {
     f[l] = own_f[l].as<uint32_t>();
   }
   coarse_one_cta = mg_coarse_fits(dims.back());
-  sweeps_fit.assign(L, 0);
-  for (size_t l = 1; l + 1 < L; l++) sweeps_fit[l] = mg_sweeps_fit(dims[l]) ? 1 : 0;
   return PYRO_OK;
 }
 
@@ -196,7 +194,7 @@ cudaError_t Multigrid::vcycles(int cycles, cudaStream_t st) {
   if ((e = tick(MG_PREPARE)) != cudaSuccess) return e;
   auto M = [&](int l) { return meta[l].as<uint8_t>(); };
   auto sm = [&](int l) -> cudaError_t {  // two red-black iterations, omega 1
-    if (sweeps_fit[l]) {
+    if (l > 0 && mg_sweeps_pay(dims[l], 4)) {
       cudaError_t e2 = launch_mg_sweeps(dims[l], h[l], b[l], M(l), phi[l], 2, 1.0f, 0, bc_mode,
                                         false, st);
       return e2 == cudaSuccess ? tick(MG_PASS_MID, 4) : e2;
@@ -299,8 +297,9 @@ cudaError_t Multigrid::vcycle_sym(cudaStream_t st, DevBuf* bphi, DevBuf* bphi2, 
     return e2 == cudaSuccess ? tick(MG_PASS_MID, 2 * n) : e2;
   };
   for (int l = 0; l < nl - 1; l++) {
-    if (sweeps_fit[l] && (e = sweeps(l, 0)) != cudaSuccess) return e;
-    for (int it = 0; it < sym_sweeps(l) && !sweeps_fit[l]; it++)
+    const bool one = l > 0 && mg_sweeps_pay(dims[l], 2 * sym_sweeps(l));
+    if (one && (e = sweeps(l, 0)) != cudaSuccess) return e;
+    for (int it = 0; it < sym_sweeps(l) && !one; it++)
       for (int c = 0; c < 2; c++) {
         e = (fuse && l == 0 && it == 0 && c == 0)
                 ? launch_mg_pass_first(dims[0], h[0], b[0], lo ? bb[0].p : nullptr, M(0), P(0), 0,
@@ -338,8 +337,9 @@ cudaError_t Multigrid::vcycle_sym(cudaStream_t st, DevBuf* bphi, DevBuf* bphi2, 
                                  dims[l + 1], M(l + 1), st);
     if (e == cudaSuccess) e = tick(l == 0 ? MG_PROLONG_L0 : MG_PROLONG_MID);
     if (e != cudaSuccess) return e;
-    if (sweeps_fit[l] && (e = sweeps(l, 1)) != cudaSuccess) return e;
-    for (int it = 0; it < sym_sweeps(l) && !sweeps_fit[l]; it++)
+    const bool one = l > 0 && mg_sweeps_pay(dims[l], 2 * sym_sweeps(l));
+    if (one && (e = sweeps(l, 1)) != cudaSuccess) return e;
+    for (int it = 0; it < sym_sweeps(l) && !one; it++)
       for (int c = 1; c >= 0; c--) {
         e = (fuse && lo && l == 0 && it == sym_sweeps(0) - 1 && c == 0)
                 ? launch_mg_pass_last_f32(dims[0], h[0], B(0), M(0), P(0), phi[0], 0, kSymOmega,

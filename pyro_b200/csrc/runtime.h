@@ -103,7 +103,6 @@ struct Multigrid {
   std::vector<DevBuf> meta;   // per-cell neighbour mask (k_mgf.cu)
   std::vector<DevBuf> wq;     // 64 x prolongation weight sums (vcycle_sym, levels < last)
   bool coarse_one_cta = false;
-  std::vector<char> sweeps_fit;  // levels whose sweeps run as one cluster launch
   float* stats = nullptr;  // device, for mg_resid
 
   // direct_max == 0: the reference rule; else the deep rule.
