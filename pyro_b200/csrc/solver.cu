@@ -406,9 +406,10 @@ __global__ void __launch_bounds__(VT) k_update_p(Cells c, M mk, float* __restric
 // ---- the CG vector kernels, W cells per thread and step
 // One cell per thread and step keeps 13 to 21 bytes in flight per cell and
 // spends most of its instructions on addresses; W consecutive cells are one
-// vector access per array.  The dot products then add a thread's W cells
-// before the next step's, an order that depends on the grid's size alone, so
-// solves still repeat bit for bit.
+// vector access per array (element by element where the caller's array is not
+// aligned for it).  The dot products then add a thread's W cells before the
+// next step's, an order that depends on the grid's size alone, so solves repeat
+// bit for bit, whatever the arrays' addresses.
 // Measured on 256^3 cells: q = A p 110 -> 60 us, the direction 55 -> 32, the
 // dots 59 -> 50, the solution and residual 88 -> 86; MGPCG to 1e-6 13.3 ->
 // 12.4 ms.
@@ -420,6 +421,16 @@ __device__ __forceinline__ void ldw(const float* p, float (&v)[W]) {
   } else {
     const float2 t = *reinterpret_cast<const float2*>(p);
     v[0] = t.x, v[1] = t.y;
+  }
+}
+// VEC false: of an array at any 4-byte alignment
+template <bool VEC, int W>
+__device__ __forceinline__ void ldw(const float* p, float (&v)[W]) {
+  if constexpr (VEC) {
+    ldw(p, v);
+  } else {
+#pragma unroll
+    for (int j = 0; j < W; j++) v[j] = __ldg(p + j);
   }
 }
 template <int W>
@@ -435,8 +446,9 @@ __device__ __forceinline__ uint32_t ldm(const uint8_t* m) {
 #define CHUNK_LOOP(i, W) \
   for (int i = (blockIdx.x * VT + threadIdx.x) * (W); i < c.n; i += gridDim.x * VT * (W))
 
-// (A v) of the W cells from i on (in one row), with their masks and values.
-template <int W>
+// (A v) of the W cells from i on (in one row), with their masks and values;
+// VEC: p is aligned to W floats.
+template <bool VEC, int W>
 __device__ __forceinline__ void applyw(const Cells& c, double ih2, const float* __restrict__ p,
                                        const uint8_t* __restrict__ meta, int i, int bc_mode,
                                        float (&v)[W], uint32_t& mw, double (&out)[W]) {
@@ -444,11 +456,11 @@ __device__ __forceinline__ void applyw(const Cells& c, double ih2, const float* 
   int x, y, z;
   c.coords(i, x, y, z);
   float yp[W], ym[W], zp[W], zm[W];
-  ldw(p + i, v);
-  ldw(p + (y + 1 < ny ? i + sy : i), yp);
-  ldw(p + (y > 0 ? i - sy : i), ym);
-  ldw(p + (z + 1 < nz ? i + sz : i), zp);
-  ldw(p + (z > 0 ? i - sz : i), zm);
+  ldw<VEC>(p + i, v);
+  ldw<VEC>(p + (y + 1 < ny ? i + sy : i), yp);
+  ldw<VEC>(p + (y > 0 ? i - sy : i), ym);
+  ldw<VEC>(p + (z + 1 < nz ? i + sz : i), zp);
+  ldw<VEC>(p + (z > 0 ? i - sz : i), zm);
   const float xl = __ldg(p + (x > 0 ? i - 1 : i)), xr = __ldg(p + (x + W < nx ? i + W : i));
   mw = ldm<W>(meta + i);
   const int fyz = (y == ny - 1) + (bc_mode == 0 ? (z == 0) + (z == nz - 1) : 0);
@@ -484,7 +496,7 @@ __global__ void __launch_bounds__(VT) k_apply_dot_w(Cells c, double ih2,
     float v[W], o[W];
     double a[W];
     uint32_t mw;
-    applyw(c, ih2, p, mk.m, i, bc_mode, v, mw, a);
+    applyw<true>(c, ih2, p, mk.m, i, bc_mode, v, mw, a);
 #pragma unroll
     for (int j = 0; j < W; j++) {
       const bool fluid = !((mw >> (8 * j)) & 0x40u);
@@ -496,9 +508,10 @@ __global__ void __launch_bounds__(VT) k_apply_dot_w(Cells c, double ih2,
   block_add_d(sh, pq, sc, SC_PQ);
 }
 
-// k_resid<MetaMask> for rows of a multiple of W cells; phi and b aligned to W
-// floats (256^3 cells: 106 -> 66 us).
-template <int W>
+// k_resid<MetaMask> for rows of a multiple of W cells.  phi and b are the
+// caller's; VEC: both aligned to W floats (256^3 cells: 106 -> 66 us, 79
+// unaligned).
+template <int W, bool VEC>
 __global__ void __launch_bounds__(VT) k_resid_w(Cells c, double ih2, const float* __restrict__ phi,
                                                 const float* __restrict__ b, MetaMask mk,
                                                 int bc_mode, float* __restrict__ r,
@@ -511,8 +524,8 @@ __global__ void __launch_bounds__(VT) k_resid_w(Cells c, double ih2, const float
     float v[W], bi[W], o[W];
     double a[W];
     uint32_t mw;
-    ldw(b + i, bi);
-    applyw(c, ih2, phi, mk.m, i, bc_mode, v, mw, a);
+    ldw<VEC>(b + i, bi);
+    applyw<VEC>(c, ih2, phi, mk.m, i, bc_mode, v, mw, a);
 #pragma unroll
     for (int j = 0; j < W; j++) {
       o[j] = 0.0f;
@@ -629,16 +642,16 @@ __global__ void __launch_bounds__(VT) k_update_p4(Cells c, MetaMask mk, float* _
 }
 
 // The form of each vector kernel for a grid: vector accesses where the cells
-// (q = A p: the rows) divide by them.
+// (q = A p and the residual: the rows) divide by them.
 inline auto apply_dot_kernel(Dims3 d) {
   return d.nx % 4 == 0 ? k_apply_dot_w<4>
                        : d.nx % 2 == 0 ? k_apply_dot_w<2> : k_apply_dot<MetaMask>;
 }
 inline auto resid_kernel(Dims3 d, const float* phi, const float* b) {
   const uintptr_t at = reinterpret_cast<uintptr_t>(phi) | reinterpret_cast<uintptr_t>(b);
-  return d.nx % 4 == 0 && at % 16 == 0
-             ? k_resid_w<4>
-             : d.nx % 2 == 0 && at % 8 == 0 ? k_resid_w<2> : k_resid<MetaMask>;
+  if (d.nx % 4 == 0) return at % 16 == 0 ? k_resid_w<4, true> : k_resid_w<4, false>;
+  if (d.nx % 2 == 0) return at % 8 == 0 ? k_resid_w<2, true> : k_resid_w<2, false>;
+  return k_resid<MetaMask>;
 }
 inline auto dots_kernel(Dims3 d) { return d.cells() % 4 == 0 ? k_dots4 : k_dots<MetaMask>; }
 inline auto update_p_kernel(Dims3 d) {

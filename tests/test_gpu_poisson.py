@@ -309,3 +309,31 @@ def test_cg_vector_kernel_forms(lib, dims, offset):
     assert np.linalg.norm((got - x)[fl]) <= 1e-3 * np.linalg.norm(x[fl])
     assert not host(buf[offset + b.size:]).any() and not host(buf[:offset]).any()
     ps.close()
+
+
+@pytest.mark.parametrize("dims", [(24, 30, 18), (26, 30, 18), (27, 29, 31)])
+@pytest.mark.parametrize("mode", [_abi.SOLVER_MGPCG, _abi.SOLVER_MGPCG_BF16])
+def test_cg_solve_does_not_depend_on_alignment(lib, dims, mode):
+    """The solution and right-hand side at every 4-byte alignment: the same
+    iterations, residuals and solution, bit for bit (the sums' order is the
+    grid's)."""
+    import torch
+
+    from pyro_b200.poisson import PoissonSolver, poisson_case
+    nx, ny, nz = dims
+    f, b = poisson_case(nx, ny, nz, seed=nx, solid=0.05, edge=(1, 3))
+    start = np.random.default_rng(3).normal(0, 0.1, b.size).astype(np.float32)
+    ps = PoissonSolver((nx, ny, nz), 0.1, 0)
+    fd = dev(f)
+    torch.cuda.synchronize()
+    ps.set_flags(fd.data_ptr())
+    out = []
+    for po, bo in ((0, 0), (1, 0), (0, 1), (2, 2), (3, 1)):
+        phi, bd = (torch.zeros(b.size + 4, dtype=torch.float32, device="cuda") for _ in range(2))
+        phi[po:po + b.size] = dev(start)
+        bd[bo:bo + b.size] = dev(b.reshape(-1))
+        torch.cuda.synchronize()
+        info = ps.solve(bd[bo:].data_ptr(), phi[po:].data_ptr(), mode, 1e-5, 100)
+        out.append((info.iterations, info.rel_resid, host(phi[po:po + b.size]).tobytes()))
+    assert all(o == out[0] for o in out), [o[:2] for o in out]
+    ps.close()
