@@ -136,8 +136,14 @@ inline Cells cells_of(Dims3 d) {
   return Cells{L3{d.nx, d.ny, d.nz}, FastDiv((uint32_t)d.nx), FastDiv((uint32_t)(d.nx * d.ny)),
                (int)d.cells()};
 }
-#define CELL_LOOP(i) \
-  for (int i = blockIdx.x * VT + threadIdx.x; i < c.n; i += gridDim.x * VT)
+// The loops' indices are unsigned: a grid has fewer than 2^31 cells, and a step
+// past the last one stays below 2^32.
+#define STRIDE_LOOP(i, n, step)                                                      \
+  for (uint32_t i##_ = (blockIdx.x * VT + threadIdx.x) * (step); i##_ < (uint32_t)(n); \
+       i##_ += gridDim.x * VT * (step))                                              \
+    if (const int i = (int)i##_; true)
+#define CELL_LOOP(i) STRIDE_LOOP(i, c.n, 1u)
+static_assert((1ull << 31) + 2ull * 4 * VT * RED_MAXB < (1ull << 32), "");
 
 // The thread's cells of the grid-stride loop in order, CG_U at a time: the
 // loads of a group (ld(cell, slot)) are all issued before any is used
@@ -151,17 +157,17 @@ constexpr int CG_U = 4;
 constexpr int XR_U = 2;
 template <int U = CG_U, typename LD, typename USE>
 __device__ __forceinline__ void cells_grouped(const Cells& c, LD ld, USE use) {
-  const int s = gridDim.x * VT;
-  int i = blockIdx.x * VT + threadIdx.x;
-  for (; i + (U - 1) * s < c.n; i += U * s) {
+  const uint32_t s = gridDim.x * VT, n = (uint32_t)c.n;
+  uint32_t i = blockIdx.x * VT + threadIdx.x;
+  for (; i + (U - 1) * s < n; i += U * s) {
 #pragma unroll
-    for (int u = 0; u < U; u++) ld(i + u * s, u);
+    for (int u = 0; u < U; u++) ld((int)(i + u * s), u);
 #pragma unroll
-    for (int u = 0; u < U; u++) use(i + u * s, u);
+    for (int u = 0; u < U; u++) use((int)(i + u * s), u);
   }
-  for (; i < c.n; i += s) {
-    ld(i, 0);
-    use(i, 0);
+  for (; i < n; i += s) {
+    ld((int)i, 0);
+    use((int)i, 0);
   }
 }
 
@@ -443,8 +449,7 @@ __device__ __forceinline__ uint32_t ldm(const uint8_t* m) {
   if constexpr (W == 4) return __ldg(reinterpret_cast<const uint32_t*>(m));
   else return __ldg(reinterpret_cast<const uint16_t*>(m));
 }
-#define CHUNK_LOOP(i, W) \
-  for (int i = (blockIdx.x * VT + threadIdx.x) * (W); i < c.n; i += gridDim.x * VT * (W))
+#define CHUNK_LOOP(i, W) STRIDE_LOOP(i, c.n, (uint32_t)(W))
 
 // (A v) of the W cells from i on (in one row), with their masks and values;
 // VEC: p is aligned to W floats.
@@ -704,12 +709,12 @@ __global__ void k_roll(double* sc) {
 // 71 -> 23 us (before: a cell per thread, an atomic per 32 cells).
 __global__ void __launch_bounds__(VT) k_flag_hash(int n, const uint32_t* __restrict__ f,
                                                   unsigned long long* out) {
-  const int st = gridDim.x * VT;
+  const uint32_t st = gridDim.x * VT;
   unsigned long long h = 0;
-  for (int i0 = blockIdx.x * VT + threadIdx.x; i0 < n; i0 += 4 * st) {
+  for (uint32_t i0 = blockIdx.x * VT + threadIdx.x; i0 < (uint32_t)n; i0 += 4 * st) {
     uint32_t v[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) v[k] = (long)i0 + (long)k * st < n ? __ldg(f + i0 + k * st) : 0u;
+    for (int k = 0; k < 4; k++) v[k] = i0 + k * st < (uint32_t)n ? __ldg(f + i0 + k * st) : 0u;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       if (v[k] != 1u) continue;
