@@ -967,6 +967,13 @@ TraceBind bind(const PyroRenderParams& R, const void* vol, const void* sol, cons
 // none, mapping the memory again cost 3 ms of a 36 ms frame); null where the
 // pool cannot be made.
 constexpr uint64_t RAY_POOL_KEEP = 256ull << 20;
+
+// The calls below are no stream's work: they neither fail nor break a capture.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 cudaMemPool_t ray_pool() {
   constexpr int MAX_DEV = 64;
   static std::mutex mu;
@@ -975,6 +982,7 @@ cudaMemPool_t ray_pool() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEV) return nullptr;
   std::lock_guard<std::mutex> lock(mu);
   if (!pools[dev]) {
+    RelaxedCapture relaxed;
     cudaMemPoolProps pr = {};
     pr.allocType = cudaMemAllocationTypePinned;
     pr.location.type = cudaMemLocationTypeDevice;

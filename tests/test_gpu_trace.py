@@ -323,6 +323,37 @@ def test_renderer_frame_vs_oracle_chain(lib):
     assert abs(img.sum() - want.sum()) <= 3e-2 * np.abs(want).sum()
 
 
+FIRST_PASS_IN_A_CAPTURE = """
+import sys
+import numpy as np, torch
+import test_gpu_trace as T
+P, d = T._glowing_frame(24, 40, 20, seed=11)
+rp = T._abi.PyroRenderParams.from_rows(T._rp_rows(P, 32, 20, 2, 7, True))
+b, lvd = T._bind(d), (12, 20, 10)
+A, B = T._half_empty((10, 20, 12, 4)), T._half_empty((10, 20, 12, 4))
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    T.render.lightvol(rp, *T._args(b), lvd, A, B, rays=4,
+                      stream=torch.cuda.current_stream().cuda_stream)
+g.replay()
+a = T._bits(T.host(A)).copy()
+T.render.lightvol(rp, *T._args(b), lvd, A, B, rays=4)
+sys.exit(0 if np.array_equal(a, T._bits(T.host(A))) else 3)
+"""
+
+
+def test_first_pass_of_a_process_under_capture(lib):
+    """A process whose first pass is captured (the scratch pool is made then)."""
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([root, os.path.join(root, "tests")]))
+    r = subprocess.run([sys.executable, "-c", FIRST_PASS_IN_A_CAPTURE], cwd=root, env=env,
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+
+
 def test_passes_under_stream_capture(lib):
     """The caches and the camera rays, with the scratch memory their launches
     take, captured into a CUDA graph: a replay gives the eager calls' bits."""
