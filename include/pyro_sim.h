@@ -541,6 +541,12 @@ int pyro_k_render_trace(const PyroRenderParams* rp, const void* vol,
                         const void* lvB, uint32_t lx, uint32_t ly, uint32_t lz,
                         const void* gE, uint32_t gres, float* accum,
                         void* stream);
+/* The three passes above lay out their volumes anew for their rays, in scratch
+ * memory (8 bytes per cell, trace 16 more per cache cell) from a pool per
+ * device that keeps up to 256 MB between launches; where the memory cannot be
+ * had, a pass reads the bound volumes: the same bits, slower.  trim gives back
+ * what no launch uses, on every device. */
+int pyro_render_trim(void);
 
 /* ---- frame development (src/post.rs:25-160, CPU code in the reference) --- */
 /* The tracer's accumulation image `accum` (w*h float4: radiance sums and

@@ -419,6 +419,11 @@ int pyro_k_mg_coarse_sym(uint32_t nx, uint32_t ny, uint32_t nz, float h, const f
              "pyro_k_mg_coarse_sym");
 }
 
+int pyro_render_trim(void) {
+  clear_error();
+  return ret(ray_pool_trim(), "pyro_render_trim");
+}
+
 int pyro_k_render_pack(const PyroParams* params_dev, uint32_t nx, uint32_t ny, uint32_t nz,
                        const float* s0, const float* s1, const float* sol,
                        const uint32_t* flags, const float* u, const float* v, const float* w,

@@ -964,9 +964,13 @@ TraceBind bind(const PyroRenderParams& R, const void* vol, const void* sol, cons
 
 // Memory for the launches' scratch: a pool of its own per device that keeps at
 // most RAY_POOL_KEEP bytes between frames (with the default pool, which keeps
-// none, mapping the memory again cost 3 ms of a 36 ms frame); null where the
-// pool cannot be made.
+// none, mapping the memory again cost 3 ms of a 36 ms frame).  It is given back
+// when the last renderer closes (pyro_render_trim) and when an allocation of
+// the library fails.
 constexpr uint64_t RAY_POOL_KEEP = 256ull << 20;
+constexpr int MAX_DEV = 64;
+std::mutex ray_pool_mu;
+cudaMemPool_t ray_pools[MAX_DEV] = {};
 
 // The calls below are no stream's work: they neither fail nor break a capture.
 struct RelaxedCapture {
@@ -974,14 +978,13 @@ struct RelaxedCapture {
   RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
   ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
+
+// The current device's pool; null where it cannot be made.
 cudaMemPool_t ray_pool() {
-  constexpr int MAX_DEV = 64;
-  static std::mutex mu;
-  static cudaMemPool_t pools[MAX_DEV] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEV) return nullptr;
-  std::lock_guard<std::mutex> lock(mu);
-  if (!pools[dev]) {
+  std::lock_guard<std::mutex> lock(ray_pool_mu);
+  if (!ray_pools[dev]) {
     RelaxedCapture relaxed;
     cudaMemPoolProps pr = {};
     pr.allocType = cudaMemAllocationTypePinned;
@@ -994,16 +997,20 @@ cudaMemPool_t ray_pool() {
       return nullptr;
     }
     cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    pools[dev] = p;
+    ray_pools[dev] = p;
   }
-  return pools[dev];
+  return ray_pools[dev];
 }
 
 }  // namespace
 
-// Gives the kept memory back (an allocation elsewhere failed).
-void ray_pool_trim() {
-  if (cudaMemPool_t p = ray_pool()) cudaMemPoolTrimTo(p, 0);
+cudaError_t ray_pool_trim() {
+  std::lock_guard<std::mutex> lock(ray_pool_mu);
+  RelaxedCapture relaxed;
+  cudaError_t e = cudaSuccess;
+  for (cudaMemPool_t p : ray_pools)
+    if (p && e == cudaSuccess) e = cudaMemPoolTrimTo(p, 0);
+  return e;
 }
 
 namespace {

@@ -69,12 +69,12 @@ cudaError_t launch_render_ecells(const PyroParams* P, Dims3 d, const void* vol, 
 size_t render_cdf_scratch_bytes(long n);
 cudaError_t launch_render_cdf(long n, const float* ecell, float* cdf, void* scratch,
                               cudaStream_t st);
+// Gives back the memory that the path tracer's scratch pools keep and no launch
+// uses, on every device.
+cudaError_t ray_pool_trim();
 // The volume path tracer (k_trace.cu) on the packed volumes: camera rays
 // into accum, the two light caches, and the caches' separable blur (radius
 // 1 .. render_blur_max_radius()).
-// Gives back the memory that the renderer's scratch pool keeps on the current
-// device.
-void ray_pool_trim();
 cudaError_t launch_render_trace(const PyroRenderParams& R, const void* vol, const void* sol,
                                 const void* vel, const float* bricks, const float* lut,
                                 const float* ecdf, const void* lvA, const void* lvB, int lx,
@@ -115,8 +115,6 @@ cudaError_t launch_mg_resid_m(Dims3 d, float h, const float* p, const float* b,
                               const uint8_t* meta, int bc_mode, float* stats, cudaStream_t st);
 cudaError_t launch_mg_resid(Dims3 d, float h, const float* p, const float* b, const uint32_t* f,
                             int bc_mode, float* stats, cudaStream_t st);
-// Whole coarsest-level solve in one CTA (shared memory); returns
-// cudaErrorInvalidValue when the level does not fit.
 // `iters` smoother sweeps (both colours, red first or black first) on a level
 // that fits a thread-block cluster, in one launch; equal to launch_mg_pass /
 // launch_mg_pass_bf16 once per colour, bit for bit.
@@ -125,6 +123,8 @@ bool mg_sweeps_pay(Dims3 d, int passes);  // fits, and is faster than a launch p
 cudaError_t launch_mg_sweeps(Dims3 d, float h, const void* b, const uint8_t* meta, void* p,
                              int iters, float omega, int black_first, int bc_mode, bool bf16,
                              cudaStream_t st);
+// Whole coarsest-level solve in one cluster launch (shared memory);
+// cudaErrorInvalidValue when the level does not fit.
 bool mg_coarse_fits(Dims3 d);
 cudaError_t launch_mg_coarse(Dims3 d, float h, const float* b, const uint32_t* f, float* p,
                              int iters, float omega, int bc_mode, cudaStream_t st);

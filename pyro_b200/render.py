@@ -18,6 +18,8 @@ from __future__ import annotations
 
 import ctypes
 import math
+import threading
+import weakref
 from typing import Optional, Sequence
 
 import numpy as np
@@ -164,6 +166,25 @@ def frame_plan(cache: bool, spp: int):
     return steps
 
 
+# The renderers alive; the passes' scratch memory is given back with the last.
+_alive = 0
+_alive_lock = threading.RLock()
+
+
+def _opened() -> None:
+    global _alive
+    with _alive_lock:
+        _alive += 1
+
+
+def _closed() -> None:
+    global _alive
+    with _alive_lock:
+        _alive -= 1
+        if _alive == 0:
+            _abi.call("pyro_render_trim")
+
+
 class Renderer:
     """Renderer::new / Renderer::render (src/render.rs:100-447) for one
     simulation: owns the light caches, their blur temporaries, the colour
@@ -190,6 +211,16 @@ class Renderer:
         self.lut = torch.from_numpy(color.build_lut()).to(dev)
         self.accum = torch.zeros((self.h * self.w, 4), dtype=torch.float32, device=dev)
         torch.cuda.synchronize()
+        _opened()
+        self._final = weakref.finalize(self, _closed)
+        self._final.atexit = False
+
+    def close(self) -> None:
+        """Drops the device buffers; called when the object is collected."""
+        if self._final.alive:
+            for n in ("lvA", "lvB", "t1", "t2", "gE", "gtmp", "lut", "accum"):
+                setattr(self, n, None)
+            self._final()
 
     def render(self, sim, frame: int, spp: int) -> np.ndarray:
         """One frame: the mean radiance per pixel, (h, w, 3) float32."""

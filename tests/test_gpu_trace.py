@@ -354,6 +354,36 @@ def test_first_pass_of_a_process_under_capture(lib):
     assert r.returncode == 0, r.stderr[-2000:]
 
 
+def test_scratch_is_given_back_with_the_last_renderer(lib):
+    """The pool keeps its memory between frames and renderers, and gives it back
+    when the last renderer closes."""
+    import gc
+
+    gc.collect()
+    assert render._alive == 0
+    sc = Scene.load(os.path.join(SCENES, "pool_small_8cm.toml"))
+    sc.render.width, sc.render.height = 24, 16
+    sim = Sim(sc)
+    rs = [render.Renderer(sc, sim, lv_rays=1, gr_rays=1, ground_res=8) for _ in range(2)]
+    for r in rs:
+        r.render(sim, 0, 1)
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    f0 = free()
+    rs[0].close()
+    rs[0].close()
+    assert free() == f0
+    rs.pop()            # collected without a call
+    del r
+    gc.collect()
+    assert render._alive == 0
+    assert free() - f0 >= 8 * np.prod(sim.dims)
+    sim.close()
+
+
 def test_passes_under_stream_capture(lib):
     """The caches and the camera rays, with the scratch memory their launches
     take, captured into a CUDA graph: a replay gives the eager calls' bits."""
