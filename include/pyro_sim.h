@@ -543,10 +543,12 @@ int pyro_k_render_trace(const PyroRenderParams* rp, const void* vol,
                         void* stream);
 /* The three passes above lay out their volumes anew for their rays, in scratch
  * memory (8 bytes per cell, trace 16 more per cache cell) from a pool per
- * device that keeps up to 256 MB between launches; where the memory cannot be
- * had, a pass reads the bound volumes: the same bits, slower.  trim gives back
- * what no launch uses, on every device. */
+ * device that keeps up to 256 MB between launches.  trim gives back what no
+ * launch uses, on every device.  scratch_limit sets the most that one launch of
+ * the calling thread takes (none at first); past it, or where the memory
+ * cannot be had, a pass reads the bound volumes: the same bits, slower. */
 int pyro_render_trim(void);
+int pyro_render_scratch_limit(uint64_t bytes);
 
 /* ---- frame development (src/post.rs:25-160, CPU code in the reference) --- */
 /* The tracer's accumulation image `accum` (w*h float4: radiance sums and

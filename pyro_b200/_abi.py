@@ -235,6 +235,7 @@ SIGNATURES = {
     "pyro_k_render_lightground": [_P, _P, _P, _P, _P, _P, _P, _U32, _U32, _P, _P],
     "pyro_k_render_blur": [_P, _P, _U32, _U32, _U32, _U32, _U32, _P],
     "pyro_render_trim": [],
+    "pyro_render_scratch_limit": [_U64],
     "pyro_k_render_trace": [_P, _P, _P, _P, _P, _P, _P, _P, _P, _U32, _U32, _U32, _P, _U32, _P,
                             _P],
     "pyro_conv3_forward": [_P, _I, _I, _I, _I, _I, _P, _I, _P, _I, _P, _I, _P],

@@ -424,6 +424,12 @@ int pyro_render_trim(void) {
   return ret(ray_pool_trim(), "pyro_render_trim");
 }
 
+int pyro_render_scratch_limit(uint64_t bytes) {
+  clear_error();
+  ray_scratch_limit(bytes);
+  return PYRO_OK;
+}
+
 int pyro_k_render_pack(const PyroParams* params_dev, uint32_t nx, uint32_t ny, uint32_t nz,
                        const float* s0, const float* s1, const float* sol,
                        const uint32_t* flags, const float* u, const float* v, const float* w,

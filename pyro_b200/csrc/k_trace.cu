@@ -200,7 +200,7 @@ struct TraceBind {
 //    temperature, smoke and heat release from vol, and both light caches are
 //    one 16-byte gather.  24 gathers a step instead of 40.
 //  * PLAIN: from the bound volumes (when the scratch memory, 8 bytes per cell
-//    and 16 per cache cell, cannot be had).
+//    and 16 per cache cell, cannot be had or is past pyro_render_scratch_limit).
 // Packing costs 24 bytes per cell of traffic (4 us on 80 x 160 x 80 cells);
 // measured there: lightvol 18.0 -> 11.3 ms, lightground 13.3 -> 7.5 ms (with the
 // guide and the fetch ahead below), 8 camera samples at 1280 x 720 9.7 -> 8.2 ms, 2 path-traced
@@ -1002,6 +1002,9 @@ cudaMemPool_t ray_pool() {
   return ray_pools[dev];
 }
 
+// The most scratch memory a launch of this thread takes.
+thread_local uint64_t ray_scratch_most = ~0ull;
+
 }  // namespace
 
 cudaError_t ray_pool_trim() {
@@ -1012,6 +1015,8 @@ cudaError_t ray_pool_trim() {
     if (p && e == cudaSuccess) e = cudaMemPoolTrimTo(p, 0);
   return e;
 }
+
+void ray_scratch_limit(uint64_t bytes) { ray_scratch_most = bytes; }
 
 namespace {
 
@@ -1024,7 +1029,7 @@ struct RayScratch {
   explicit RayScratch(cudaStream_t s) : st(s) {}
   // false when the memory cannot be had (the error is cleared)
   bool alloc(size_t n) {
-    cudaMemPool_t pool = ray_pool();
+    cudaMemPool_t pool = n <= ray_scratch_most ? ray_pool() : nullptr;
     if (pool && cudaMallocFromPoolAsync(&p, n, pool, st) == cudaSuccess) return true;
     p = nullptr;
     cudaGetLastError();

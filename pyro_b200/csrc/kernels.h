@@ -70,8 +70,10 @@ size_t render_cdf_scratch_bytes(long n);
 cudaError_t launch_render_cdf(long n, const float* ecell, float* cdf, void* scratch,
                               cudaStream_t st);
 // Gives back the memory that the path tracer's scratch pools keep and no launch
-// uses, on every device.
+// uses, on every device; and the most scratch memory that a launch of the
+// calling thread takes.
 cudaError_t ray_pool_trim();
+void ray_scratch_limit(uint64_t bytes);
 // The volume path tracer (k_trace.cu) on the packed volumes: camera rays
 // into accum, the two light caches, and the caches' separable blur (radius
 // 1 .. render_blur_max_radius()).

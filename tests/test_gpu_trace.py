@@ -354,6 +354,32 @@ def test_first_pass_of_a_process_under_capture(lib):
     assert r.returncode == 0, r.stderr[-2000:]
 
 
+@pytest.mark.parametrize("cache", [True, False])
+@pytest.mark.parametrize("dims", [(24, 40, 20), (9, 21, 5)])
+def test_unpacked_forms_give_the_same_bits(lib, cache, dims):
+    """The passes with no scratch memory, from the bound volumes, against the
+    packed forms, motion blur and depth of field included: the same bits."""
+    P, d = _glowing_frame(*dims, seed=13)
+    rp = _abi.PyroRenderParams.from_rows(_rp_rows(P, 40, 24, 4, 5, cache, aperture=0.02))
+    b = _bind(d)
+    lvd, gres = tuple((n + 1) // 2 for n in dims), 16
+    out = []
+    try:
+        for limit in (2 ** 64 - 1, 0):
+            assert lib.pyro_render_scratch_limit(limit) == 0
+            A, B = _half_empty((*lvd[::-1], 4)), _half_empty((*lvd[::-1], 4))
+            G = _half_empty((1, gres, gres, 4))
+            acc = torch.zeros((40 * 24, 4), dtype=torch.float32, device="cuda")
+            render.lightvol(rp, *_args(b), lvd, A, B, rays=6)
+            render.lightground(rp, *_args(b), gres, G, rays=6)
+            render.trace(rp, *_args(b), A, B, lvd, G, gres, acc)
+            out.append([host(t).tobytes() for t in (A, B, G, acc)])
+            assert host(acc).any()
+    finally:
+        assert lib.pyro_render_scratch_limit(2 ** 64 - 1) == 0
+    assert out[0] == out[1]
+
+
 def test_scratch_is_given_back_with_the_last_renderer(lib):
     """The pool keeps its memory between frames and renderers, and gives it back
     when the last renderer closes."""
