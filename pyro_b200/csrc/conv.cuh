@@ -1,5 +1,5 @@
-// conv.cuh — activation layout and epilogue shared by the convolution kernels
-// (k_conv.cu, k_conv3.cu).
+// conv.cuh — activation layout of the learned stage (net.cu) and the epilogue
+// shared by its convolution kernels (k_conv.cu, k_conv3.cu).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -9,8 +9,11 @@ namespace {
 
 using bf16 = __nv_bfloat16;
 
-// Activation layout: C a multiple of 8 -> C / 8 planes of [V][8 channels];
-// otherwise [V][C].  Element offset of channel c of voxel v:
+// Activation layout: a tensor of C channels over V voxels with C a multiple of
+// 8 is stored as C / 8 planes of [V][8 channels] (a plane is one 16-byte chunk
+// per voxel, so a TMA box along x reads long contiguous rows); other channel
+// counts (the 2-channel input, 1-channel gradients) as [V][C].  Element offset
+// of channel c of voxel v:
 __device__ __forceinline__ size_t act_off(size_t v, int c, int C, size_t V) {
   return (C & 7) ? v * C + c : ((size_t)(c >> 3) * V + v) * 8 + (c & 7);
 }

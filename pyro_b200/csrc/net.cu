@@ -14,13 +14,13 @@
 #include <vector>
 
 #include "common.cuh"
+#include "conv.cuh"
 #include "net.h"
 
 namespace pyro {
 
 namespace {
 
-using bf16 = __nv_bfloat16;
 constexpr int NT = 256;
 constexpr int MAX_VOLS = 64;
 // device scalars: weighted pressure loss, gradient sum of squares, sum of
@@ -85,15 +85,6 @@ __device__ __forceinline__ void plane_split(size_t i, size_t V, size_t& v, int& 
     p = (int)(i / V);
     v = i - (size_t)p * V;
   }
-}
-
-// Activation layout: a tensor of C channels over V voxels with C a multiple
-// of 8 is stored as C / 8 planes of [V][8 channels] (a plane is one 16-byte
-// chunk per voxel, so a TMA box along x reads long contiguous rows); other
-// channel counts (the 2-channel input, 1-channel gradients) as [V][C].
-// Element offset of channel c of voxel v:
-__device__ __forceinline__ size_t act_off(size_t v, int c, int C, size_t V) {
-  return (C & 7) ? v * C + c : ((size_t)(c >> 3) * V + v) * 8 + (c & 7);
 }
 
 inline unsigned blocks_for(size_t n) {

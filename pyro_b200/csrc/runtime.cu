@@ -133,7 +133,7 @@ int Multigrid::init(Dims3 d0, float h0, int bc, size_t direct_max) {
     b[l] = own_b[l].as<float>();
     f[l] = own_f[l].as<uint32_t>();
   }
-  coarse_one_cta = mg_coarse_fits(dims.back());
+  coarse_in_cluster = mg_coarse_fits(dims.back());
   return PYRO_OK;
 }
 
@@ -147,7 +147,7 @@ size_t Multigrid::device_bytes() const {
 
 cudaError_t Multigrid::smooth(int l, int iters, bool coarse, cudaStream_t st) {
   float om = coarse ? 1.6f : 1.0f;
-  if (coarse && coarse_one_cta)
+  if (coarse && coarse_in_cluster)
     return launch_mg_coarse(dims[l], h[l], b[l], f[l], phi[l], iters, om, bc_mode, st);
   for (int it = 0; it < iters; it++)
     for (int c = 0; c < 2; c++) {
@@ -320,7 +320,7 @@ cudaError_t Multigrid::vcycle_sym(cudaStream_t st, DevBuf* bphi, DevBuf* bphi2, 
   int lc = nl - 1;
   if (direct) {
     if ((e = direct->apply(st, B(lc), P(lc), lo)) != cudaSuccess) return e;
-  } else if (coarse_one_cta) {
+  } else if (coarse_in_cluster) {
     e = lo ? launch_mg_coarse_sym_bf16(dims[lc], h[lc], B(lc), f[lc], P(lc), 80, 1.6f, bc_mode, st)
            : launch_mg_coarse_sym(dims[lc], h[lc], (const float*)B(lc), f[lc], (float*)P(lc), 80,
                                   1.6f, bc_mode, st);

@@ -102,7 +102,7 @@ struct Multigrid {
   std::vector<DevBuf> phi2;   // ping-pong partner of phi on every level
   std::vector<DevBuf> meta;   // per-cell neighbour mask (k_mgf.cu)
   std::vector<DevBuf> wq;     // 64 x prolongation weight sums (vcycle_sym, levels < last)
-  bool coarse_one_cta = false;
+  bool coarse_in_cluster = false;
   float* stats = nullptr;  // device, for mg_resid
 
   // direct_max == 0: the reference rule; else the deep rule.

@@ -32,16 +32,6 @@ __device__ __forceinline__ uint64_t smem_desc(const void* base, int rows) {
   return start | (lbo << 16) | (sbo << 32) | (1ull << 46);  // version 1, no swizzle
 }
 
-// Descriptor with an explicit leading-byte offset (distance between the two
-// 8-element K halves of a 16-wide K step); core matrices along M/N 128 B
-// apart.
-__device__ __forceinline__ uint64_t smem_desc_lbo(const void* base, uint32_t lbo_bytes) {
-  uint64_t start = (smem_u32(base) >> 4) & 0x3FFFull;
-  uint64_t lbo = ((uint64_t)lbo_bytes >> 4) & 0x3FFFull;
-  uint64_t sbo = (128ull >> 4) & 0x3FFFull;
-  return start | (lbo << 16) | (sbo << 32) | (1ull << 46);
-}
-
 // Instruction descriptor, kind::f16: D f32, A and B bf16, both K-major.
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) |
@@ -143,7 +133,7 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* mbar, uint32_t bytes) {
                : "memory");
 }
 
-// TMA tiled loads global -> this CTA's shared memory, completing on `mbar`.
+// TMA tiled load global -> this CTA's shared memory, completing on `mbar`.
 // Coordinates are element indices, innermost first; out-of-range boxes are
 // zero-filled.  The innermost coordinate times the element size must be a
 // multiple of 16 bytes.
@@ -156,24 +146,6 @@ __device__ __forceinline__ void tma_load_5d(void* dst, const void* tmap, int c0,
       "r"(smem_u32(mbar))
       : "memory");
 }
-__device__ __forceinline__ void tma_load_4d(void* dst, const void* tmap, int c0, int c1, int c2,
-                                            int c3, uint64_t* mbar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(c2), "r"(c3),
-      "r"(smem_u32(mbar))
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(void* dst, const void* tmap, int c0, int c1, int c2,
-                                            uint64_t* mbar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(mbar))
-      : "memory");
-}
-
 // 32 lanes x 16 columns of 32-bit TMEM into 16 registers per thread.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   uint32_t r[16];
@@ -187,24 +159,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]);
-}
-
-// 32 lanes x 32 columns of 32-bit TMEM into 32 registers per thread.
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int j = 0; j < 32; j++) v[j] = __uint_as_float(r[j]);
 }
 
 }  // namespace umma
