@@ -11,7 +11,8 @@
 //                    B[n = ci][k]                = W[co][tap][ci]
 //   backward (weight) A[m = (tap, ci)][k = voxel] = x[voxel + tap][ci]
 //                    B[n = co][k = voxel]        = dy[voxel][co]   (split over K;
-//                    channel counts that k_wgrad.cu does not take)
+//                    channel counts and alignments that k_wgrad.cu does not
+//                    take, and gradients with sums that are not finite)
 //
 // Activations are BF16 in planes of 8 channels, [C / 8][volume][z][y][x][8]
 // (C a multiple of 8; [volume][z][y][x][C] otherwise); a tap

@@ -15,7 +15,7 @@
 //                 on the CPU; the three scales run side by side, each in
 //                 place in a buffer of its own
 //   box_h, box_v  the same filters from global memory, for images whose rows
-//                 do not fit the shared memory (wider than ~16,000 pixels)
+//                 do not fit the shared memory (wider than 9,016 pixels)
 //   final         glare mix, ACES fit, sRGB, dither and 8-bit quantisation
 //                 (post.rs:47-88)
 //
@@ -166,7 +166,7 @@ constexpr int GV_DEPTH = 4;       // groups in flight
 constexpr size_t GLARE_SMEM = 220 * 1024;
 
 // words per row of glare_h: the row r + 1 pixels in, rounded up to 3 mod 32
-// words so that the 12 chains read different banks
+// words so that the 6 chains read different banks
 __host__ __device__ __forceinline__ int gh_pitch(int w, int r) {
   const int n = 3 * (w + r + 1);
   return (n + 28) / 32 * 32 + 3;

@@ -73,8 +73,10 @@ def test_select_rejects_bad_arguments():
 
 
 @pytest.mark.parametrize("h,w", [(1, 1), (5, 3), (3, 64), (33, 250), (122, 75), (61, 640),
-                                 (5, 4096),    # the widest rows in shared memory
-                                 (3, 17000)])  # past them: filters from global memory
+                                 (5, 4096),
+                                 (3, 9016),    # the widest rows in shared memory
+                                 (3, 9017),    # past them: filters from global memory
+                                 (3, 17000)])
 def test_glare_filters_bit_for_bit(h, w):
     """The linear image after the glare mix, bit for bit the restatement's
     running sums, for rows and columns shorter than a filter, ragged groups
