@@ -47,12 +47,13 @@
 //
 // Measured on 160 x 320 x 160 voxels against the form this replaces (output
 // channels as the MMA's 128 rows, of which 16 to 64 were used, and three
-// shifted copies of x), in us: 16 -> 16 773 -> 244, 48 -> 16 1990 -> 598; on
-// 80 x 160 x 80, 96 -> 32 522 -> 320; the data gradient 16 -> 48 on two 128^3
-// volumes 1411 -> 370.  What bounds it now: the MMAs' issue
-// (48 -> 16: 54 MMAs of 48 cycles per 512 voxels and group are 0.44 ms at
-// 1.9 GHz; copying the input with cp.async from four warps measured 684 us
-// against 598 with the boxes).
+// shifted copies of x), in us: 16 -> 16 773 -> 258, 48 -> 16 1990 -> 631; on
+// 80 x 160 x 80, 96 -> 32 522 -> 382 with the up-sampled store; the data
+// gradient 16 -> 48 on two 128^3 volumes 1411 -> 401 (the test for sums that
+// are not finite costs 5 to 8 % of it).  What bounds it now: the boxes' rows
+// (16 cycles for 160 bytes: 48 -> 16 0.59 ms at 1.9 GHz) ahead of the MMAs'
+// issue (54 of 48 cycles per 512 voxels and group, 0.44 ms); copying the input
+// with cp.async from four warps was slower (684 us against 598).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
