@@ -1009,10 +1009,12 @@ thread_local uint64_t ray_scratch_most = ~0ull;
 
 cudaError_t ray_pool_trim() {
   std::lock_guard<std::mutex> lock(ray_pool_mu);
-  RelaxedCapture relaxed;
   cudaError_t e = cudaSuccess;
-  for (cudaMemPool_t p : ray_pools)
-    if (p && e == cudaSuccess) e = cudaMemPoolTrimTo(p, 0);
+  for (cudaMemPool_t p : ray_pools) {
+    if (!p || e != cudaSuccess) continue;
+    RelaxedCapture relaxed;
+    e = cudaMemPoolTrimTo(p, 0);
+  }
   return e;
 }
 

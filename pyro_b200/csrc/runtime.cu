@@ -19,7 +19,7 @@ int DevBuf::alloc(size_t n) {
   cudaError_t e = cudaMalloc(&p, n);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    ray_pool_trim();
+    if (ray_pool_trim() != cudaSuccess) cudaGetLastError();
     e = cudaMalloc(&p, n);
   }
   if (e != cudaSuccess) {
