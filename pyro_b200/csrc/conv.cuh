@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cuda_bf16.h>
+#include <stdint.h>
 
 namespace pyro {
 namespace {
@@ -32,7 +33,9 @@ struct ConvEpi {
   int up, fx, fy, fz, fV;
   __device__ void operator()(int m, int col, const float (&v)[16]) const {
     if (m < 0 || m >= V) return;
-    if (out_bf16 && (Nout & 15) == 0) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(out_bf16) |
+                         reinterpret_cast<uintptr_t>(mask) | reinterpret_cast<uintptr_t>(bias);
+    if (out_bf16 && (Nout & 15) == 0 && (at & 15) == 0) {
       // 16 channels of one row: 32 contiguous bytes, two 16-byte stores
       float a[16];
 #pragma unroll

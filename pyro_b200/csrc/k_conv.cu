@@ -76,8 +76,7 @@ template <int N, class Load, class Epi>
 __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(Load ld, Epi ep, int ksteps_total,
                                                        int ksteps_per_cta, int* err,
                                                        const int* only_if) {
-  pdl_trigger();
-  pdl_wait();
+  pdl_wait();  // no early trigger: the next launch's CTAs may allocate TMEM before they wait
   if (only_if && *only_if == 0) return;
   constexpr int NCOLS = N <= 32 ? 32 : (N <= 64 ? 64 : 128);
   __shared__ __align__(1024) uint8_t sA[2][128 * 32];
@@ -506,12 +505,17 @@ cudaError_t conv3_wgrad_gather(const bf16* x, int Cin, const bf16* dy, int Cout,
 }
 
 // Direct convolution for the shapes k_conv_direct covers (2 -> 16 and
-// 16 -> 1 channels); cudaErrorInvalidValue for others.
+// 16 -> 1 channels); cudaErrorInvalidValue for others and for tensors off the
+// boundary of its accesses (x: a voxel's 4 bytes, a plane's 16; BF16 output of
+// 16 channels: 16).
 bool conv3_direct_fits(int C, int Cout) { return (C == 2 && Cout == 16) || (C == 16 && Cout == 1); }
 
 cudaError_t conv3_direct(const bf16* x, int C, int nx, int ny, int nz, int nb, const bf16* w,
                          int Cout, const float* bias, int relu, bf16* y_bf16, float* y_f32,
                          cudaStream_t st) {
+  if (reinterpret_cast<uintptr_t>(x) % (C == 2 ? 4 : 16) ||
+      (!y_f32 && Cout % 8 == 0 && reinterpret_cast<uintptr_t>(y_bf16) % 16))
+    return cudaErrorInvalidValue;
   Vol g{nx, ny, nz, nb};
   auto blocks = [&](int dv) {
     return (unsigned)(((long)((nx + dv - 1) / dv) * ny * nz * nb + 255) / 256);

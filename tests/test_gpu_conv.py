@@ -349,3 +349,40 @@ def test_backward_weight_error_bounded_by_the_gather(lib, Cin, Cout, dims):
         assert rc == 0, lib.pyro_last_error()
         errs.append(((dw - ref).norm() / ref.norm()).item())
     assert errs[0] <= errs[1], errs
+
+
+@pytest.mark.parametrize("Cin,Cout", [(8, 16), (3, 32)])
+def test_gather_unaligned(lib, Cin, Cout):
+    """The gather GEMM's outputs, mask and bias at 2- or 4-byte alignment: the
+    bits of the aligned call."""
+    nz, ny, nx = 5, 6, 7
+    x, w, b = _tensors(1, Cin, nz, ny, nx, Cout, 61)
+    dy, _, _ = _tensors(1, Cin, nz, ny, nx, 1, 62)
+    act, w2, _ = _tensors(1, Cout, nz, ny, nx, Cin, 63)
+    n = nz * ny * nx * Cout
+    xc, wk, dc, wk2, ac = _cl(x), _wk(w), _cl(dy), _wk(w2), _cl(act).reshape(-1)
+    outs = []
+    for o in (0, 1, 3):
+        y = torch.zeros(n + 8, dtype=torch.bfloat16, device="cuda")
+        dx, m = torch.zeros_like(y), torch.zeros_like(y)
+        bb = torch.zeros(Cout + 4, device="cuda")
+        bb[o:o + Cout] = b
+        m[o:o + n] = ac
+        assert lib.pyro_conv3_forward(ptr(xc), Cin, nx, ny, nz, 1, ptr(wk), Cout, ptr(bb[o:]), 1,
+                                      ptr(y[o:]), 0, None) == 0, lib.pyro_last_error()
+        # channels swapped: Cin gradients into Cout masked ones
+        assert lib.pyro_conv3_backward_data(ptr(dc), Cin, nx, ny, nz, 1, ptr(wk2), Cout,
+                                            ptr(m[o:]), ptr(dx[o:]), 0, None) == 0
+        outs.append((y[o:o + n].clone(), dx[o:o + n].clone()))
+    for y, dx in outs[1:]:
+        assert torch.equal(y, outs[0][0]) and torch.equal(dx, outs[0][1])
+
+
+def test_direct_unaligned_is_refused(lib):
+    """Tensors off the boundary of the direct kernel's accesses."""
+    x = torch.zeros(4 * 5 * 6 * 16 + 8, dtype=torch.bfloat16, device="cuda")
+    w, y = torch.zeros_like(x), torch.zeros(4096, device="cuda")
+    for C, Cout, xo, yo in ((16, 1, 1, 0), (16, 1, 4, 0), (2, 16, 1, 0), (2, 16, 0, 1)):
+        rc = lib.pyro_conv3_forward(ptr(x[xo:]), C, 6, 5, 4, 1, ptr(w), Cout, None, 0,
+                                    ptr(y.bfloat16()[yo:]) if yo else ptr(y), 0, None)
+        assert rc < 0
