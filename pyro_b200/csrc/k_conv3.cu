@@ -47,10 +47,10 @@
 //
 // Measured on 160 x 320 x 160 voxels against the form this replaces (output
 // channels as the MMA's 128 rows, of which 16 to 64 were used, and three
-// shifted copies of x), in us: 16 -> 16 773 -> 258, 48 -> 16 1990 -> 631; on
+// shifted copies of x), in us: 16 -> 16 773 -> 255, 48 -> 16 1990 -> 612; on
 // 80 x 160 x 80, 96 -> 32 522 -> 382 with the up-sampled store; the data
-// gradient 16 -> 48 on two 128^3 volumes 1411 -> 401 (the test for sums that
-// are not finite costs 5 to 8 % of it).  What bounds it now: the boxes' rows
+// gradient 16 -> 48 on two 128^3 volumes 1411 -> 404 (the test for sums that
+// are not finite costs 2 to 8 % of it).  What bounds it now: the boxes' rows
 // (16 cycles for 160 bytes: 48 -> 16 0.59 ms at 1.9 GHz) ahead of the MMAs'
 // issue (54 of 48 cycles per 512 voxels and group, 0.44 ms); copying the input
 // with cp.async from four warps was slower (684 us against 598).
@@ -90,8 +90,8 @@ struct C3Geom {
 // max of `top` and |v|, NaN if one is NaN
 __device__ __forceinline__ float max_abs(const float (&v)[16], float top) {
 #pragma unroll
-  for (int e = 0; e < 16; e++)
-    asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(fabsf(v[e])));
+  for (int e = 0; e < 16; e += 2)
+    asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(top) : "f"(fabsf(v[e])), "f"(fabsf(v[e + 1])));
   return top;
 }
 
