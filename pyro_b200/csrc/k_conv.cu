@@ -589,8 +589,9 @@ int pyro_conv3_forward(const void* x, int C, int nx, int ny, int nz, int nb, con
     if ((rc = wt.alloc((size_t)Cout * 27 * C * 2)) != PYRO_OK) return rc;
     e = conv3_prep_weights((const bf16*)w, Cout, C, 0, wt.as<bf16>(), st);
     if (e == cudaSuccess)
-      e = conv3_tma((const bf16*)x, C, false, nx, ny, nz, nb, wt.as<bf16>(), Cout, bias, relu, nullptr,
-                    y_f32 ? nullptr : (bf16*)y, y_f32 ? (float*)y : nullptr, err.as<int>(), st);
+      e = conv3_tma((const bf16*)x, C, false, nx, ny, nz, nb, wt.as<bf16>(), Cout, bias, relu,
+                    nullptr, y_f32 ? nullptr : (bf16*)y, y_f32 ? (float*)y : nullptr,
+                    err.as<int>(), st);
     return finish(e, err, st, "pyro_conv3_forward");
   }
   e = conv3_forward((const bf16*)x, C, nx, ny, nz, nb, (const bf16*)w, Cout, bias, relu,

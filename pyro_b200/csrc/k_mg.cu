@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(256) k_mg_resid(Lvl d, float h2, const float* 
 // A ghost plane is not overwritten while it is read: a neighbour sends in
 // pass p + 1 only after it has all of this CTA's cells of pass p, and a thread
 // here sends a cell after it has loaded that cell's ghost neighbour; in pass
-// p + 1 itself this CTA reads the other colour of the ghosts.  The last pass sends nothing, so no store is in flight to a CTA
-// that ends.
+// p + 1 itself this CTA reads the other colour of the ghosts.  The last pass
+// sends nothing, so no store is in flight to a CTA that ends.
 //
 // The two colours live in separate arrays, indexed by the reference
 // smoother's own numbering q = hx + hxn (y + ny z), x = 2 hx + ((y + z + c) &

@@ -652,8 +652,8 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
     // pk holds the shifts of the last layer's gradient, then the first's input
     const int pack = L.cout == 1 ? 1 : L.cin == 2 ? 2 : 0;
     e = conv3_wgrad_tma(pack == 2 ? pk.as<bf16>() : xs, L.cin, pack == 1 ? pk.as<bf16>() : gs,
-                        L.cout, pack, g.nx, g.ny, g.nz, g.nb, wsum.as<double>() + w_off[l], E, bad + l,
-                        st);
+                        L.cout, pack, g.nx, g.ny, g.nz, g.nb, wsum.as<double>() + w_off[l], E,
+                        bad + l, st);
     if (e != cudaSuccess) return e;
     float* db = G + n_w + b_off[l];
     if (L.cout % 8 == 0)
@@ -667,8 +667,9 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
   auto bd = [&](const DevBuf& dz, int l, NetVol g, const DevBuf* act, DevBuf& dx) -> cudaError_t {
     const NetLayer& L = NET_SPEC[l];
     const bool one = L.cout == 1;
-    return conv3_tma(one ? pk.as<bf16>() : dz.as<bf16>(), L.cout, one, g.nx, g.ny, g.nz, g.nb, wb(l), L.cin, nullptr, 0, act ? act->as<bf16>() : nullptr,
-                     dx.as<bf16>(), nullptr, E, st, nullptr, true);
+    return conv3_tma(one ? pk.as<bf16>() : dz.as<bf16>(), L.cout, one, g.nx, g.ny, g.nz, g.nb, wb(l),
+                     L.cin, nullptr, 0, act ? act->as<bf16>() : nullptr, dx.as<bf16>(), nullptr, E,
+                     st, nullptr, true);
   };
   NET_CU(conv3_pack_grad(g9.as<bf16>(), v.nx, v.ny, v.nz, v.nb, pk.as<bf16>(), st));
   NET_CU(wg(d0, g9, 8, v));
