@@ -72,20 +72,36 @@ __device__ __forceinline__ void st_bf(uint8_t* s, uint32_t off, bf16 v) {
   *reinterpret_cast<bf16*>(s + off) = v;
 }
 
+// TMEM of a block that computes tiles one after another (allocated once: a
+// block that has given up its permit may not allocate again).
+constexpr int gemm_cols(int N) { return N <= 32 ? 32 : (N <= 64 ? 64 : 128); }
+template <int N>
+__device__ uint32_t gemm_alloc() {
+  __shared__ uint32_t tslot;
+  if (threadIdx.x < 32) {
+    umma::tmem_alloc(&tslot, gemm_cols(N));
+    umma::tmem_relinquish();
+  }
+  umma::fence_before();
+  __syncthreads();
+  umma::fence_after();
+  return tslot;
+}
+template <int N>
+__device__ void gemm_free(uint32_t tbase) {
+  umma::fence_before();
+  __syncthreads();
+  if (threadIdx.x < 32) umma::tmem_dealloc(tbase, gemm_cols(N));
+}
+
+// One tile: rows m0 .. m0 + 127, K steps k0 .. k1 - 1; the whole block calls.
+// False when a wait ran out: the block computes no further tile.
 template <int N, class Load, class Epi>
-__global__ void __launch_bounds__(GEMM_THREADS) k_gemm(Load ld, Epi ep, int ksteps_total,
-                                                       int ksteps_per_cta, int* err,
-                                                       const int* only_if) {
-  pdl_wait();  // no early trigger: the next launch's CTAs may allocate TMEM before they wait
-  if (only_if && *only_if == 0) return;
-  constexpr int NCOLS = N <= 32 ? 32 : (N <= 64 ? 64 : 128);
+__device__ bool gemm_tile(const Load& ld, const Epi& ep, uint32_t tbase, int m0, int k0, int k1,
+                          int* err) {
   __shared__ __align__(1024) uint8_t sA[2][128 * 32];
   __shared__ __align__(1024) uint8_t sB[2][N * 32];
   __shared__ __align__(8) uint64_t mbar[2];
-  __shared__ uint32_t tslot;
-  const int m0 = blockIdx.x * 128;
-  const int k0 = blockIdx.y * ksteps_per_cta;
-  const int k1 = min(k0 + ksteps_per_cta, ksteps_total);
   const int nks = max(k1 - k0, 0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -93,14 +109,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(Load ld, Epi ep, int kste
     umma::mbar_init(&mbar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) {
-    umma::tmem_alloc(&tslot, NCOLS);
-    umma::tmem_relinquish();
-  }
-  umma::fence_before();
   __syncthreads();
-  umma::fence_after();
-  const uint32_t tbase = tslot;
   constexpr uint32_t IDESC = umma::idesc_bf16(128, N);
   bool ok = true;
   for (int i = 0; i < nks; i++) {
@@ -116,8 +125,9 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(Load ld, Epi ep, int kste
       umma::mma_commit(&mbar[s]);
     }
   }
-  if (nks > 0 && !umma::mbar_wait_bounded(&mbar[(nks - 1) & 1], ((nks - 1) >> 1) & 1))
-    ok = false;
+  // both barriers' last phases: nothing arrives on them any more
+  for (int i = max(nks - 2, 0); i < nks; i++)
+    if (!umma::mbar_wait_bounded(&mbar[i & 1], (i >> 1) & 1)) ok = false;
   umma::fence_after();
   const bool all_ok = __syncthreads_and(ok) != 0;
   if (all_ok && nks > 0) {
@@ -129,9 +139,27 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(Load ld, Epi ep, int kste
     }
   }
   if (!all_ok && threadIdx.x == 0) atomicExch(err, 1);
+  // the sums are read and the barriers done with before the next tile
   umma::fence_before();
   __syncthreads();
-  if (warp == 0) umma::tmem_dealloc(tbase, NCOLS);
+  if (all_ok && threadIdx.x == 0) {
+    umma::mbar_inval(&mbar[0]);
+    umma::mbar_inval(&mbar[1]);
+  }
+  __syncthreads();
+  return all_ok;
+}
+
+template <int N, class Load, class Epi>
+__global__ void __launch_bounds__(GEMM_THREADS) k_gemm(Load ld, Epi ep, int ksteps_total,
+                                                       int ksteps_per_cta, int* err,
+                                                       const int* only_if) {
+  pdl_wait();  // no early trigger: the next launch's CTAs may allocate TMEM before they wait
+  if (only_if && *only_if == 0) return;
+  const int k0 = blockIdx.y * ksteps_per_cta;
+  const uint32_t tbase = gemm_alloc<N>();
+  gemm_tile<N>(ld, ep, tbase, blockIdx.x * 128, k0, min(k0 + ksteps_per_cta, ksteps_total), err);
+  gemm_free<N>(tbase);
 }
 
 // ---------------------------------------------------------------- loaders
@@ -262,6 +290,35 @@ struct WgradEpi {
     }
   }
 };
+
+// The weight gradients of a network's layers that have bad[l] set, one launch
+// for all: the blocks share a layer's tiles, layer after layer (a launch per
+// layer that ends at once took 7 us each).
+constexpr int WG_N = 64;  // output channels at most
+struct WgradJobs {
+  WgradLoad ld[NET_LAYERS];
+  WgradEpi ep[NET_LAYERS];
+  int ksteps[NET_LAYERS], per[NET_LAYERS];
+};
+__global__ void __launch_bounds__(GEMM_THREADS)
+    k_wgrad_gathers(const __grid_constant__ WgradJobs J, const int* __restrict__ bad, int* err) {
+  pdl_wait();
+  int any = 0;
+  for (int l = 0; l < NET_LAYERS; l++) any |= bad[l];
+  if (!any) return;
+  const uint32_t tbase = gemm_alloc<WG_N>();
+  bool ok = true;
+  for (int l = 0; l < NET_LAYERS; l++) {
+    if (!bad[l]) continue;
+    const int mt = (J.ep[l].M + 127) / 128, splits = (J.ksteps[l] + J.per[l] - 1) / J.per[l];
+    for (int t = blockIdx.x; ok && t < mt * splits; t += gridDim.x) {
+      const int k0 = t / mt * J.per[l];
+      ok = gemm_tile<WG_N>(J.ld[l], J.ep[l], tbase, t % mt * 128, k0,
+                           min(k0 + J.per[l], J.ksteps[l]), err);
+    }
+  }
+  gemm_free<WG_N>(tbase);
+}
 
 template <int N, class Load, class Epi>
 cudaError_t gemm_launch(dim3 grid, const Load& ld, const Epi& ep, int ksteps_total,
@@ -485,6 +542,22 @@ int conv3_gather_steps(int Cin, long V) {
   // split K so that the grid covers the GPU a few times over
   const long splits = std::max(1l, std::min(ksteps, (148 * 8) / std::max(mt, 1l)));
   return (int)((ksteps + splits - 1) / splits);
+}
+
+cudaError_t conv3_wgrad_gathers(const WgradJob (&jobs)[NET_LAYERS], const int* bad, int* err,
+                                cudaStream_t st) {
+  WgradJobs J;
+  for (int l = 0; l < NET_LAYERS; l++) {
+    const WgradJob& j = jobs[l];
+    const NetLayer& L = NET_SPEC[l];
+    const long V = (long)j.v.voxels();
+    static_assert(NET_SPEC[5].cout == WG_N, "");
+    J.ld[l] = WgradLoad{j.x, j.g, Vol{j.v.nx, j.v.ny, j.v.nz, j.v.nb}, L.cin, L.cout, WG_N};
+    J.ep[l] = WgradEpi{j.dw, 27 * L.cin, L.cout};
+    J.ksteps[l] = (int)((V + 15) / 16);
+    J.per[l] = conv3_gather_steps(L.cin, V);
+  }
+  return launch_pdl(k_wgrad_gathers, dim3(148 * 8), dim3(GEMM_THREADS), 0, st, J, bad, err);
 }
 
 // dw[co][tap][ci] += sum_voxels dy[v][co] x[v + tap][ci]  (dw FP32).

@@ -640,12 +640,9 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
       (double)w_res, (double)out_scale, w_res > 0.0f ? res.as<float>() : nullptr, g9.as<bf16>());
   NET_CU(cudaGetLastError());
   int* bad = reinterpret_cast<int*>(S + SC_VOL + 2 * MAX_VOLS);  // cleared by forward
-  struct Wg {
-    const bf16 *x, *g;
-    NetVol v;
-  } layers[NET_LAYERS];
+  WgradJob layers[NET_LAYERS];
   auto wg = [&](const DevBuf& x, const DevBuf& dz, int l, NetVol g) -> cudaError_t {
-    layers[l] = Wg{x.as<bf16>(), dz.as<bf16>(), g};
+    layers[l] = WgradJob{x.as<bf16>(), dz.as<bf16>(), g, G + w_off[l]};
     const NetLayer& L = NET_SPEC[l];
     const bf16 *xs = x.as<bf16>(), *gs = dz.as<bf16>();
     cudaError_t e;
@@ -702,11 +699,7 @@ int PyroNet::loss_backward(const float* b, const uint32_t* flags, const float* p
   k_wgrad_out<<<dim3(64, NET_LAYERS), NT, 0, st>>>(WOff(w_off), wsum.as<double>(), bad, G);
   NET_CU(cudaGetLastError());
   // layers with sums that are not finite, from the gather GEMM
-  for (int l = 0; l < NET_LAYERS; l++) {
-    const Wg& a = layers[l];
-    NET_CU(conv3_wgrad_gather(a.x, NET_SPEC[l].cin, a.g, NET_SPEC[l].cout, a.v.nx, a.v.ny, a.v.nz,
-                              a.v.nb, G + w_off[l], E, bad + l, st));
-  }
+  NET_CU(conv3_wgrad_gathers(layers, bad, E, st));
   return PYRO_OK;
 }
 

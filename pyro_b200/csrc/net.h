@@ -27,6 +27,15 @@
 
 namespace pyro {
 
+constexpr int NET_LAYERS = 9;
+struct NetLayer {
+  int cin, cout, level, relu;
+};
+// conv1 .. conv9 in order
+constexpr NetLayer NET_SPEC[NET_LAYERS] = {{2, 16, 0, 1},  {16, 16, 0, 1}, {16, 32, 1, 1},
+                                           {32, 32, 1, 1}, {32, 64, 2, 1}, {64, 64, 2, 1},
+                                           {96, 32, 1, 1}, {48, 16, 0, 1}, {16, 1, 0, 0}};
+
 struct NetVol {
   int nx, ny, nz, nb;
   size_t voxels() const { return (size_t)nx * ny * nz * nb; }
@@ -94,14 +103,14 @@ cudaError_t conv3_pack_grad(const __nv_bfloat16* src, int nx, int ny, int nz, in
 cudaError_t conv3_pack_input(const __nv_bfloat16* src, int nx, int ny, int nz, int nb,
                              __nv_bfloat16* dst, cudaStream_t st);
 
-constexpr int NET_LAYERS = 9;
-struct NetLayer {
-  int cin, cout, level, relu;
+// The same of the network's layers with bad[l] set (device), in one launch.
+struct WgradJob {
+  const __nv_bfloat16 *x, *g;
+  NetVol v;
+  float* dw;
 };
-// conv1 .. conv9 in order
-constexpr NetLayer NET_SPEC[NET_LAYERS] = {{2, 16, 0, 1},  {16, 16, 0, 1}, {16, 32, 1, 1},
-                                           {32, 32, 1, 1}, {32, 64, 2, 1}, {64, 64, 2, 1},
-                                           {96, 32, 1, 1}, {48, 16, 0, 1}, {16, 1, 0, 0}};
+cudaError_t conv3_wgrad_gathers(const WgradJob (&jobs)[NET_LAYERS], const int* bad, int* err,
+                                cudaStream_t st);
 
 }  // namespace pyro
 

@@ -137,6 +137,41 @@ def test_forward_is_its_layers_bit_for_bit(lib, dims, nb):
     assert np.array_equal(host(phi), host(want))
 
 
+def test_gradients_of_layers_behind_one_that_is_not_finite(lib):
+    """A NaN weight of conv6 makes its output channel 0 (ReLU) and, on the way
+    back, one channel of conv5's gradient NaN.  The layers above, and conv5's
+    other channels, have the gradients of the network whose channel is switched
+    off instead; everything below is not finite.  FP32 sums in another order:
+    1e-3 of a layer's largest gradient."""
+    dims, nb, h, co, t, ci = (12, 16, 20), 2, 0.05, 7, 13, 21
+    b, flags, phi_t = _case(12, nb, dims)
+    bd, fd, pd = _dev_case(b, flags, phi_t)
+    nz, ny, nx = dims
+    grads = []
+    for bad in (False, True):
+        net, p = _net(13, w_phi=1.0, w_res=0.0)
+        ws, bs = L.unpack(p)
+        ws, bs = [w.copy() for w in ws], [v.copy() for v in bs]
+        if bad:
+            ws[5][co, t, ci] = np.nan
+        else:
+            ws[5][co], bs[5][co] = 0.0, -1.0
+        net.set_params(L.pack(ws, bs).astype(np.float32), net.get_params()[1])
+        net.set_loss(1.0, 0.0)
+        loss, g = net.loss_grad(bd.data_ptr(), fd.data_ptr(), pd.data_ptr(), (nx, ny, nz), nb, h)
+        assert np.isfinite(loss)
+        grads.append(L.unpack(g.astype(np.float64))[0])
+    want, got = grads
+    keep6, keep5 = np.arange(64) != co, np.arange(64) != ci
+    for l, rows in ((8, None), (7, None), (6, None), (5, keep6), (4, keep5)):
+        a, e = (got[l], want[l]) if rows is None else (got[l][rows], want[l][rows])
+        assert np.isfinite(a).all(), l
+        assert np.abs(a - e).max() <= 1e-3 * np.abs(e).max(), l
+    assert not np.isfinite(got[4][ci]).any()
+    for l in range(4):
+        assert not np.isfinite(got[l]).all(), l
+
+
 @pytest.mark.parametrize("w_phi,w_res,scale", [(1.0, 0.0, 1.0), (0.3, 2.0, 2.0)])
 def test_gradient_matches_oracle_and_finite_differences(lib, w_phi, w_res, scale):
     dims, nb, h = (8, 8, 12), 2, 0.05
